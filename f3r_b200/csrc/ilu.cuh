@@ -13,6 +13,9 @@
 // (CSR::inverse_last, csr.hpp:60-65).  fp16 values, fp32 accumulation.
 #pragma once
 
+#include <algorithm>
+#include <cstring>
+#include <string>
 #include <vector>
 
 #include "device.cuh"
@@ -30,39 +33,26 @@ struct IluTri {
   __half *dinv = nullptr;  // upper only: fp16(1 / u_ii), per q
   int32_t *lvl_off = nullptr;  // row ranges (in q) of the levels, all blocks
   int32_t *blk_lvl = nullptr;  // per block: first level index (nblocks + 1)
-  int32_t *blk_pos = nullptr;  // per block: first vector position (nblocks + 1)
-  int32_t nlevels_max = 0;
-  int32_t smem_rows = 0;  // > 0: blocks occupy contiguous positions, each at most this many rows
 };
 
-// One CTA per block-Jacobi block.  The factor is stored in the order the
-// kernel visits rows (level by level within a block), so a row's data is one
-// int4 of metadata and a contiguous run of entries: two dependent loads,
-// coalesced across the threads of a level.  When the blocks occupy
-// contiguous vector positions (T.smem_rows > 0) the block's results are also
-// kept in shared memory, so a row reads the rows it depends on (all in its
-// block, written at earlier levels) from there instead of from L2.  The
-// terms are the reference's, in its order: the forward sweep by increasing
-// column, the backward sweep by decreasing column.
+// One CTA per block-Jacobi block, rows level by level; the factor stays in
+// global memory.  Used where the blocks' rows do not occupy contiguous vector
+// positions (sigma-sorted rows) or a block or row is too large for
+// k_bj_stream below.
 template <bool UPPER>
 __global__ void k_trsv_bj(IluTri T, const __half *__restrict__ in, __half *__restrict__ out,
                           const __half *__restrict__ ome) {
-  extern __shared__ __half sy[];
   const int b = blockIdx.x;
   const int l0 = T.blk_lvl[b], l1 = T.blk_lvl[b + 1];
   const float om = ome ? __half2float(*ome) : 1.0f;
-  const bool sm = T.smem_rows > 0;
-  const int32_t p0 = sm ? T.blk_pos[b] : 0;
   for (int l = l0; l < l1; l++) {
     const int r0 = T.lvl_off[l], r1 = T.lvl_off[l + 1];
     for (int q = r0 + threadIdx.x; q < r1; q += blockDim.x) {
       const int4 m = T.meta[q];
       float t = __half2float(in[m.x]);
       for (int32_t j = m.y; j < m.z; j++)
-        t = __fmaf_rn(-__half2float(T.val[j]), __half2float(sm ? sy[T.idx[j] - p0] : out[T.idx[j]]), t);
-      const __half h = UPPER ? __float2half_rn(t * __half2float(T.dinv[q])) : __float2half_rn(t);
-      out[m.x] = h;
-      if (sm) sy[m.x - p0] = h;
+        t = __fmaf_rn(-__half2float(T.val[j]), __half2float(out[T.idx[j]]), t);
+      out[m.x] = UPPER ? __float2half_rn(t * __half2float(T.dinv[q])) : __float2half_rn(t);
     }
     __syncthreads();
   }
@@ -70,15 +60,157 @@ __global__ void k_trsv_bj(IluTri T, const __half *__restrict__ in, __half *__res
   if (UPPER && ome) {
     for (int q = T.lvl_off[l0] + threadIdx.x; q < T.lvl_off[l1]; q += blockDim.x) {
       const int32_t p = T.meta[q].x;
-      out[p] = __float2half_rn(__half2float(sm ? sy[p - p0] : out[p]) * om);
+      out[p] = __float2half_rn(__half2float(out[p]) * om);
     }
   }
 }
 
-constexpr int32_t kIluSmemRows = 48 * 1024;  // fp16 results of one block in shared memory: 96 KB at most
+// ---------------------------------------------------------------------------
+// Both triangular solves of a block in one CTA, the block's vector in shared
+// memory and its factors streamed through a ring of bulk copies.
+//
+// The time of a block solve is its chain of dependency levels (137 levels of
+// 17 rows for a 64^3 27-point matrix over 112 blocks), so what counts is the
+// latency of one level.  Each factor is packed, in the order the kernel visits
+// rows, into chunks of kBjChunk bytes: the row ranges that may run in parallel
+// ("parts", a level or a piece of one), 4 bytes a row (position in the block,
+// fp16 inverse diagonal) and 4 bytes an entry (fp16 value, 16-bit position in
+// the block), padded to the part's longest row so that no lane branches.  The copy engine keeps kBjStages chunks
+// ahead of the sweep, so a level costs only shared-memory latencies; a row's
+// packed data is read one and two parts ahead, which leaves the gather of y,
+// the multiply-add chain and one barrier between two levels.  W warps sweep (one,
+// without any block barrier, where levels hold up to 32 rows on average); the
+// other warps only load and store the block's vector.
+// 64^3, 112 blocks, both factors (272 levels): 49 us, where one launch a factor
+// reading it from L2 level by level took 453 us; the solve 15.9 ms against 59.7.
+// What is left is the sweep's own chain, 0.17 us a level.
+// The in-place vector y holds the right-hand side, then L^-1 in, then the
+// result; the terms and roundings of a row are k_trsv_bj's.
+// ---------------------------------------------------------------------------
+constexpr int kBjChunk = 16384, kBjStages = 4, kBjThreads = 256, kBjMaxWarps = 8;
+constexpr int32_t kIluSmemRows = 48 * 1024;  // longest block: fp16 vector of 96 KB, 16-bit positions
+
+struct BjStream {
+  const unsigned char *chunks = nullptr;  // chunk c at c * kBjChunk
+  const int32_t *blk_chunk = nullptr;     // per block: first chunk (nblocks + 1); lower chunks, then upper ones
+  const int32_t *blk_pos = nullptr;       // per block: first vector position (nblocks + 1)
+  int32_t warps = 1;                      // sweeping warps
+  int32_t max_rows = 0;
+  size_t smem() const { return y_bytes() + (size_t)kBjStages * (kBjChunk + sizeof(uint64_t)) + 16; }
+  __host__ __device__ size_t y_bytes() const { return ((size_t)(max_rows + 1) * sizeof(__half) + 127) / 128 * 128; }
+};
+
+// Chunk: 4 words {parts, 0, 0, 0}; 2 words a part; 1 word a row; the entries,
+// from a 16-byte boundary, in groups of 4 words, a part's first groups row by
+// row, then its second ones ...: every row of a part has the part's groups.
+//   part word 0: first row word (from the chunk) | rows << 16; word 1: first group (16-byte units) | groups << 16
+//   row word: position | fp16 1/u_ii (1 in L) << 16
+//   entry word: position | fp16 -value << 16; padding entries are 0 times the zero kept behind the block's vector
+template <bool MULTI>
+__global__ void __launch_bounds__(kBjThreads) k_bj_stream(BjStream T, const __half *__restrict__ in,
+                                                          __half *__restrict__ out, const __half *__restrict__ ome,
+                                                          int *err) {
+  extern __shared__ __align__(128) unsigned char bj_smem[];
+  __half *y = reinterpret_cast<__half *>(bj_smem);
+  unsigned char *ring = bj_smem + T.y_bytes();
+  uint64_t *bars = reinterpret_cast<uint64_t *>(ring + (size_t)kBjStages * kBjChunk);
+  volatile int *gave_up = reinterpret_cast<volatile int *>(bars + kBjStages);
+  const int b = blockIdx.x;
+  const int c0 = T.blk_chunk[b], c1 = T.blk_chunk[b + 1];
+  const int32_t p0 = T.blk_pos[b], len = T.blk_pos[b + 1] - p0;
+  auto fetch = [&](int c) {
+    const int st = (c - c0) % kBjStages;
+    fence_proxy_async_smem();
+    mbar_arrive_expect_tx(&bars[st], kBjChunk);
+    bulk_g2s(ring + (size_t)st * kBjChunk, T.chunks + (size_t)c * kBjChunk, kBjChunk, &bars[st]);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kBjStages; s++) mbar_init(&bars[s], 1);
+    *gave_up = 0;
+    fence_mbar_init();
+    for (int c = c0; c < min(c1, c0 + kBjStages); c++) fetch(c);
+  }
+#pragma unroll 8
+  for (int i = threadIdx.x; i < len; i += kBjThreads) y[i] = in[p0 + i];
+  if (threadIdx.x == 0) y[len] = __ushort_as_half((unsigned short)0);  // what padding entries multiply
+  __syncthreads();
+  const int width = MULTI ? T.warps * 32 : 32;
+  const int tid = threadIdx.x;
+  if (tid < width) {
+    auto sync = [&]() {
+      if (MULTI) asm volatile("bar.sync 1, %0;" ::"r"(width) : "memory");
+      else __syncwarp();
+    };
+    int c = c0;
+    for (; c < c1; c++) {
+      const int st = (c - c0) % kBjStages;
+      const bool ok = mbar_wait_bounded(&bars[st], (uint32_t)(((c - c0) / kBjStages) & 1));
+      if (!ok) *gave_up = 1;
+      sync();
+      if (*gave_up) break;
+      const uint32_t *ch = reinterpret_cast<const uint32_t *>(ring + (size_t)st * kBjChunk);
+      const int np = ch[0];
+      const uint2 *parts = reinterpret_cast<const uint2 *>(ch + 4);
+      const uint4 *ent = reinterpret_cast<const uint4 *>(ch);
+      auto half_of = [&](uint32_t bits) { return __ushort_as_half((unsigned short)bits); };
+      // row l of part d: m its word, e its first group; stored where live
+      auto row = [&](const uint2 d, int l, uint32_t m, uint4 e, bool live) {
+        const int nr = d.x >> 16, ng = d.y >> 16;
+        float t = __half2float(y[m & 0xffffu]);
+        for (int g = 0; g < ng; g++) {
+          const uint32_t w[4] = {e.x, e.y, e.z, e.w};
+          __half v[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) v[u] = y[w[u] & 0xffffu];
+          if (g + 1 < ng) e = ent[(d.y & 0xffffu) + (g + 1) * nr + l];
+#pragma unroll
+          for (int u = 0; u < 4; u++) t = fma_vx<float>(half_of(w[u] >> 16), v[u], t);
+        }
+        if (live) y[m & 0xffffu] = __float2half_rn(t * __half2float(half_of(m >> 16)));
+      };
+      // part words are read two parts ahead, this thread's row word and first
+      // group one (threads past a part's rows repeat its last row, unstored)
+      auto lane_row = [&](const uint2 d) { return min(tid, (int)(d.x >> 16) - 1); };
+      uint2 d0 = parts[0], d1 = parts[min(1, np - 1)];
+      int l0 = lane_row(d0);
+      uint32_t m0 = ch[(d0.x & 0xffffu) + l0];
+      uint4 e0 = ent[(d0.y & 0xffffu) + l0];
+      for (int q = 0; q < np; q++) {
+        const uint2 d2 = parts[min(q + 2, np - 1)];
+        const int l1 = lane_row(d1);
+        const uint32_t m1 = ch[(d1.x & 0xffffu) + l1];
+        const uint4 e1 = ent[(d1.y & 0xffffu) + l1];
+        const int nr = d0.x >> 16;
+        row(d0, l0, m0, e0, tid < nr);
+        for (int r = tid + width; r < nr; r += width)  // a part without entries has no groups to read
+          row(d0, r, ch[(d0.x & 0xffffu) + r], ent[(d0.y & 0xffffu) + (d0.y >> 16 ? r : 0)], true);
+        sync();
+        d0 = d1;
+        d1 = d2;
+        l0 = l1;
+        m0 = m1;
+        e0 = e1;
+      }
+      // every thread is past its reads of this stage: refill it
+      if (tid == 0 && c + kBjStages < c1) fetch(c + kBjStages);
+    }
+    if (c < c1 && tid == 0) {
+      atomicCAS(err, 0, (int)DEV_TIMEOUT_TRSV);
+      // let the copies in flight land before the block's shared memory goes (bounded)
+      for (int k = c; k < min(c1, c + kBjStages); k++)
+        mbar_wait_bounded(&bars[(k - c0) % kBjStages], (uint32_t)(((k - c0) / kBjStages) & 1));
+    }
+  }
+  __syncthreads();
+  // the reference solves, then scales: hout *= ome[0] (work/src/f3r.cpp:216, 229)
+  const float om = ome ? __half2float(*ome) : 1.0f;
+  for (int i = threadIdx.x; i < len; i += kBjThreads)
+    out[p0 + i] = ome ? __float2half_rn(__half2float(y[i]) * om) : y[i];
+}
 
 struct IluDevice {
-  IluTri L, U;
+  IluTri L, U;      // where the blocks cannot be streamed
+  BjStream stream;  // max_rows > 0: the fused solve
   int32_t nblocks = 0;
   std::vector<void *> allocs;
 
@@ -135,59 +267,187 @@ struct IluDevice {
     }
   }
 
-  Status build_tri(IluTri &T, const HostCSR &M, bool upper, const std::vector<int32_t> &bptr,
-                   const std::vector<int32_t> &pos) {
-    std::vector<int32_t> order, lvl_off, blk_lvl;
-    levels(M, upper, bptr, order, lvl_off, blk_lvl, T.nlevels_max);
-    // blocks on contiguous positions (natural order) and of at most
-    // kIluSmemRows rows keep their results in shared memory
-    const int32_t nb = (int32_t)bptr.size() - 1;
-    std::vector<int32_t> bpos(nb + 1, 0);
-    bool contiguous = true;
-    int32_t maxlen = 0;
-    for (int32_t b = 0; b < nb; b++) {
-      bpos[b] = bptr[b] < bptr[b + 1] ? pos[bptr[b]] : 0;
-      maxlen = std::max(maxlen, bptr[b + 1] - bptr[b]);
-      for (int32_t i = bptr[b]; i < bptr[b + 1] && contiguous; i++) contiguous = pos[i] == bpos[b] + (i - bptr[b]);
-    }
-    T.smem_rows = (contiguous && maxlen <= kIluSmemRows) ? std::max(maxlen, 1) : 0;
-    // the factor in visiting order: fp16 values rounded once from fp64 (the
-    // reference casts CSR<double> to CSR<__half>, csr.hpp:23-25)
-    const size_t nq = order.size();
-    std::vector<int4> meta(nq);
-    std::vector<double> v, dinv;
-    std::vector<int32_t> idx;
-    v.reserve(M.val.size());
-    idx.reserve(M.idx.size());
-    if (upper) dinv.resize(nq);
+  // a factor in the order the kernels visit it: rows by block and level, a
+  // row's off-diagonal entries in processing order (increasing columns for L,
+  // decreasing for U)
+  struct TriHost {
+    std::vector<int32_t> order, lvl_off, blk_lvl, idx;
+    std::vector<int4> meta;
+    std::vector<double> val, dinv;
+  };
+  static void visit_order(TriHost &t, const HostCSR &M, bool upper, const std::vector<int32_t> &bptr,
+                          const std::vector<int32_t> &pos) {
+    int32_t nlevels = 0;
+    levels(M, upper, bptr, t.order, t.lvl_off, t.blk_lvl, nlevels);
+    const size_t nq = t.order.size();
+    t.meta.resize(nq);
+    t.val.reserve(M.val.size());
+    t.idx.reserve(M.idx.size());
+    if (upper) t.dinv.resize(nq);
     for (size_t q = 0; q < nq; q++) {
-      const int32_t i = order[q], r0 = M.rptr[i], r1 = M.rptr[i + 1];
-      meta[q].x = pos[i];
-      meta[q].y = (int32_t)idx.size();
+      const int32_t i = t.order[q], r0 = M.rptr[i], r1 = M.rptr[i + 1];
+      t.meta[q].x = pos[i];
+      t.meta[q].y = (int32_t)t.idx.size();
       if (!upper) {
         for (int32_t j = r0; j < r1 - 1; j++) {  // last entry is the unit diagonal
-          v.push_back(M.val[j]);
-          idx.push_back(pos[M.idx[j]]);
+          t.val.push_back(M.val[j]);
+          t.idx.push_back(pos[M.idx[j]]);
         }
       } else {
         for (int32_t j = r1 - 1; j > r0; j--) {  // first entry is the diagonal
-          v.push_back(M.val[j]);
-          idx.push_back(pos[M.idx[j]]);
+          t.val.push_back(M.val[j]);
+          t.idx.push_back(pos[M.idx[j]]);
         }
-        dinv[q] = 1.0 / M.val[r0];
+        t.dinv[q] = 1.0 / M.val[r0];
       }
-      meta[q].z = (int32_t)idx.size();
-      meta[q].w = 0;
+      t.meta[q].z = (int32_t)t.idx.size();
+      t.meta[q].w = 0;
     }
-    if (up(&T.meta, meta) != cudaSuccess || up(&T.idx, idx) != cudaSuccess || up(&T.lvl_off, lvl_off) != cudaSuccess ||
-        up(&T.blk_lvl, blk_lvl) != cudaSuccess || up(&T.blk_pos, bpos) != cudaSuccess)
+  }
+
+  Status upload_tri(IluTri &T, const TriHost &h, bool upper) {
+    if (up(&T.meta, h.meta) != cudaSuccess || up(&T.idx, h.idx) != cudaSuccess ||
+        up(&T.lvl_off, h.lvl_off) != cudaSuccess || up(&T.blk_lvl, h.blk_lvl) != cudaSuccess)
       return fail(F3R_ERROR_CUDA, "ILU upload failed");
-    F3R_TRY(to_half(&T.val, v));
-    if (upper) F3R_TRY(to_half(&T.dinv, dinv));
+    // fp16 values rounded once from fp64 (the reference casts CSR<double> to CSR<__half>, csr.hpp:23-25)
+    F3R_TRY(to_half(&T.val, h.val));
+    if (upper) F3R_TRY(to_half(&T.dinv, h.dinv));
     return F3R_SUCCESS;
   }
 
   Status to_half(__half **d, const std::vector<double> &v);
+  // v rounded to fp16 as the device rounds it
+  Status half_bits(std::vector<uint16_t> &h, const std::vector<double> &v) {
+    __half *d = nullptr;
+    F3R_TRY(to_half(&d, v));
+    h.resize(v.size());
+    const cudaError_t e = v.empty() ? cudaSuccess : cudaMemcpy(h.data(), d, v.size() * 2, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    allocs.pop_back();
+    return e == cudaSuccess ? F3R_SUCCESS : fail(F3R_ERROR_CUDA, "ILU values");
+  }
+
+  // Appends one factor of block b (len rows from position p0) to the block's
+  // chunks (see k_bj_stream).  false when a row does not fit a chunk.
+  static bool pack_block(std::vector<uint32_t> &out, const TriHost &t, const std::vector<uint16_t> &val,
+                         const std::vector<uint16_t> &dinv, bool upper, int32_t b, int32_t p0, int32_t len) {
+    constexpr int kWords = kBjChunk / 4;
+    auto up4 = [](int x) { return (x + 3) & ~3; };
+    struct Part {
+      std::vector<int32_t> rows;
+      int groups = 0;
+    };
+    std::vector<Part> parts;
+    auto groups_of = [&](int32_t q) { return (t.meta[q].z - t.meta[q].y + 3) / 4; };
+    int nrows = 0, closed = 0;  // rows of the chunk; entry words of its complete parts
+    auto fits = [&](int np, int nr, int entries) { return 4 + 2 * np + up4(nr + (2 * np & 2)) + 4 + entries <= kWords; };
+    auto flush = [&]() {
+      if (parts.empty()) return;
+      const size_t base = out.size();
+      out.resize(base + kWords, 0u);
+      uint32_t *c = out.data() + base;
+      const int np = (int)parts.size();
+      c[0] = (uint32_t)np;
+      int rw = 4 + 2 * np, at = up4(rw + nrows);
+      for (int q = 0; q < np; q++) {
+        const Part &pt = parts[q];
+        const int nr = (int)pt.rows.size();
+        c[4 + 2 * q] = (uint32_t)rw | ((uint32_t)nr << 16);
+        c[4 + 2 * q + 1] = (pt.groups ? (uint32_t)(at / 4) : 0u) | ((uint32_t)pt.groups << 16);
+        for (int r = 0; r < nr; r++) {
+          const int4 m = t.meta[pt.rows[r]];
+          c[rw + r] = (uint32_t)(m.x - p0) | ((upper ? (uint32_t)dinv[pt.rows[r]] : 0x3C00u) << 16);
+          for (int k = 0; k < 4 * pt.groups; k++) {
+            const int32_t j = m.y + k;
+            c[at + ((k / 4) * nr + r) * 4 + k % 4] =
+                j < m.z ? (uint32_t)(t.idx[j] - p0) | ((uint32_t)(val[j] ^ 0x8000u) << 16) : (uint32_t)len;
+          }
+        }
+        rw += nr;
+        at += 4 * nr * pt.groups;
+      }
+      parts.clear();
+      nrows = 0;
+      closed = 0;
+    };
+    for (int32_t l = t.blk_lvl[b]; l < t.blk_lvl[b + 1]; l++) {
+      bool open = false;  // this level's part in the chunk
+      for (int32_t q = t.lvl_off[l]; q < t.lvl_off[l + 1]; q++) {
+        const int g = groups_of(q);
+        if (!fits(1, 1, 4 * g)) return false;
+        if (open) {
+          Part &pt = parts.back();
+          const int ng = std::max(pt.groups, g);
+          if (!fits((int)parts.size(), nrows + 1, closed + 4 * ng * ((int)pt.rows.size() + 1))) {
+            flush();
+            open = false;
+          }
+        } else if (!fits((int)parts.size() + 1, nrows + 1, closed + 4 * g)) {
+          flush();
+        }
+        if (!open) {
+          parts.emplace_back();
+          open = true;
+        }
+        parts.back().rows.push_back(q);
+        parts.back().groups = std::max(parts.back().groups, g);
+        nrows++;
+      }
+      if (open) closed += 4 * parts.back().groups * (int)parts.back().rows.size();
+    }
+    flush();
+    return true;
+  }
+
+  // the chunks of all blocks; stream.max_rows stays 0 where the blocks do not
+  // occupy contiguous positions, or a block or row is too large
+  Status build_stream(const TriHost &l, const TriHost &u, const std::vector<int32_t> &bptr,
+                      const std::vector<int32_t> &pos) {
+    const int32_t nb = (int32_t)bptr.size() - 1;
+    std::vector<int32_t> bpos(nb + 1, 0), first(nb + 1, 0);
+    int32_t maxlen = 0;
+    for (int32_t b = 0; b < nb; b++) {
+      bpos[b] = bptr[b];
+      maxlen = std::max(maxlen, bptr[b + 1] - bptr[b]);
+      for (int32_t i = bptr[b]; i < bptr[b + 1]; i++)
+        if (pos[i] != i) return F3R_SUCCESS;
+    }
+    bpos[nb] = bptr[nb];
+    if (maxlen > kIluSmemRows) return F3R_SUCCESS;
+    std::vector<uint16_t> lv, uv, ud;
+    F3R_TRY(half_bits(lv, l.val));
+    F3R_TRY(half_bits(uv, u.val));
+    F3R_TRY(half_bits(ud, u.dinv));
+    std::vector<std::vector<uint32_t>> packed(nb);
+    int bad = 0;
+#pragma omp parallel for schedule(dynamic, 1) reduction(+ : bad)
+    for (int32_t b = 0; b < nb; b++)
+      if (!pack_block(packed[b], l, lv, ud, false, b, bpos[b], bpos[b + 1] - bpos[b]) ||
+          !pack_block(packed[b], u, uv, ud, true, b, bpos[b], bpos[b + 1] - bpos[b]))
+        bad++;
+    if (bad) return F3R_SUCCESS;
+    std::vector<uint32_t> all;
+    for (int32_t b = 0; b < nb; b++) {
+      all.insert(all.end(), packed[b].begin(), packed[b].end());
+      first[b + 1] = (int32_t)(all.size() / (kBjChunk / 4));
+      std::vector<uint32_t>().swap(packed[b]);
+    }
+    unsigned char *d = nullptr;
+    int32_t *fd = nullptr, *pd = nullptr;
+    std::vector<unsigned char> bytes(all.size() * 4);
+    std::memcpy(bytes.data(), all.data(), bytes.size());
+    if (up(&d, bytes) != cudaSuccess || up(&fd, first) != cudaSuccess || up(&pd, bpos) != cudaSuccess)
+      return fail(F3R_ERROR_OUT_OF_MEMORY, "ILU upload failed");
+    stream.chunks = d;
+    stream.blk_chunk = fd;
+    stream.blk_pos = pd;
+    stream.max_rows = std::max(maxlen, 1);
+    // warps by the mean rows of a level: one warp needs no block barrier
+    const int64_t lev = (int64_t)l.lvl_off.size() + (int64_t)u.lvl_off.size() - 2;
+    const int64_t avg = lev > 0 ? 2 * (int64_t)l.order.size() / lev : 0;
+    stream.warps = (int32_t)std::max<int64_t>(1, std::min<int64_t>(kBjMaxWarps, (avg + 31) / 32));
+    return F3R_SUCCESS;
+  }
 
   Status build(cudaStream_t, const HostCSR &Lh, const HostCSR &Uh, const std::vector<int32_t> &perm, bool permuted,
                const std::vector<int32_t> &bptr) {
@@ -197,20 +457,37 @@ struct IluDevice {
     if (permuted)
       for (int32_t s = 0; s < n; s++) pos[perm[s]] = s;
     nblocks = (int32_t)bptr.size() - 1;
-    F3R_TRY(build_tri(L, Lh, false, bptr, pos));
-    F3R_TRY(build_tri(U, Uh, true, bptr, pos));
-    // the attribute is the kernel's, shared by every solver: always the cap
-    const int cap = (int)(kIluSmemRows * sizeof(__half));
-    if (cudaFuncSetAttribute(k_trsv_bj<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap) != cudaSuccess ||
-        cudaFuncSetAttribute(k_trsv_bj<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap) != cudaSuccess)
-      return fail(F3R_ERROR_CUDA, "ILU shared-memory attribute");
-    return F3R_SUCCESS;
+    TriHost l, u;
+    visit_order(l, Lh, false, bptr, pos);
+    visit_order(u, Uh, true, bptr, pos);
+    F3R_TRY(build_stream(l, u, bptr, pos));
+    if (stream.max_rows > 0) {
+      // the attribute is the kernel's, shared by every solver: always the cap
+      BjStream cap;
+      cap.max_rows = kIluSmemRows;
+      if (cudaFuncSetAttribute(k_bj_stream<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap.smem()) !=
+              cudaSuccess ||
+          cudaFuncSetAttribute(k_bj_stream<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap.smem()) !=
+              cudaSuccess)
+        return fail(F3R_ERROR_CUDA, "ILU shared-memory attribute");
+      return F3R_SUCCESS;
+    }
+    F3R_TRY(upload_tri(L, l, false));
+    return upload_tri(U, u, true);
   }
 
-  // out = U^-1 L^-1 x (tmp holds L^-1 x); ome (nullable) scales the result
-  Status apply(cudaStream_t st, const __half *x, __half *tmp, __half *out, const __half *ome) const {
-    k_trsv_bj<false><<<nblocks, 256, (size_t)L.smem_rows * sizeof(__half), st>>>(L, x, tmp, nullptr);
-    k_trsv_bj<true><<<nblocks, 256, (size_t)U.smem_rows * sizeof(__half), st>>>(U, tmp, out, ome);
+  int launches() const { return stream.max_rows > 0 ? 1 : 2; }  // kernels of one apply
+
+  // out = U^-1 L^-1 x (tmp: scratch); ome (nullable) scales the result
+  Status apply(cudaStream_t st, const __half *x, __half *tmp, __half *out, const __half *ome, int *err) const {
+    if (nblocks == 0) return F3R_SUCCESS;
+    if (stream.max_rows > 0) {
+      if (stream.warps > 1) k_bj_stream<true><<<nblocks, kBjThreads, stream.smem(), st>>>(stream, x, out, ome, err);
+      else k_bj_stream<false><<<nblocks, kBjThreads, stream.smem(), st>>>(stream, x, out, ome, err);
+    } else {
+      k_trsv_bj<false><<<nblocks, 256, 0, st>>>(L, x, tmp, nullptr);
+      k_trsv_bj<true><<<nblocks, 256, 0, st>>>(U, tmp, out, ome);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(F3R_ERROR_CUDA, std::string("ILU trsv launch: ") + cudaGetErrorString(e));
     return F3R_SUCCESS;

@@ -958,8 +958,8 @@ template <int K> struct Engine {
     }
     if constexpr (K == 1) {
       if (p.precond == F3R_PRECOND_ILU0_BJ) {
-        F3R_TRY(S.ilu.apply(C().stream, x, w.tmp, out, scale_ome ? &w.rs->ome[0] : nullptr));
-        C().launches += 2;
+        F3R_TRY(S.ilu.apply(C().stream, x, w.tmp, out, scale_ome ? &w.rs->ome[0] : nullptr, C().err));
+        C().launches += S.ilu.launches();
       } else if (p.precond == F3R_PRECOND_ILU0_LEVEL) {
         F3R_TRY(S.ilul.apply(C().stream, x, w.tmp, out, scale_ome ? &w.rs->ome[0] : nullptr, C().err));
         C().launches += 2;

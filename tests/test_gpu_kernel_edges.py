@@ -1,0 +1,40 @@
+"""Kernels chosen by a rule on sizes, at the edges of their ranges, against the
+oracle's arithmetic or the general kernel."""
+import numpy as np
+import pytest
+import torch
+
+import f3r_b200 as F
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return F.Context(0)
+
+
+@pytest.mark.parametrize("grid,blocks,sigma", [
+    ((16, 16, 16), 1, 1), ((16, 16, 16), 7, 1), ((16, 16, 16), 4096, 1),  # one block, ragged blocks, single rows
+    ((64, 64, 1), 5, 1), ((32, 32, 16), 1, 1),                            # one and several sweeping warps
+    ((64, 32, 32), 1, 1),                                                 # longer than the streamed kernel takes
+    ((16, 16, 16), 7, 256)])                                              # blocks not contiguous
+def test_block_ilu_solve_is_the_oracles(ctx, grid, blocks, sigma):
+    """One outer step over one application of M = U^-1 L^-1 to a residual of
+    entries +-1 (its norm, a power of two, and the fp16 input are exact): x is
+    the fp16 result times one factor, rounded to fp32."""
+    A = F.stencil27(*grid, 1, 0.5).scale()
+    n = A.shape[0]
+    r, i, v = A.arrays()
+    b = np.where(F.random_uniform(3, 0.0, 1.0, n) < 0.5, -1.0, 1.0)
+    M = O.Mat.from_csr(r, i, v)
+    L, U = O.ilu0_bj(M, blocks)
+    h = (b / np.sqrt(n)).astype(np.float16)
+    want = O.trsv(U, True, O.trsv(L, False, h, prod_fma=True), prod_fma=True).astype(np.float64)
+    S = F.Solver(ctx, A, precond=F.PRECOND_ILU0_BJ, ilu_blocks=blocks, sell_sigma=sigma, m2=1, m3=0, m4=1,
+                 static_weight=1.0)
+    x = np.zeros(n)
+    S.solve(b, x, cond=lambda it, e: it >= 1)
+    c = np.dot(x, want) / np.dot(want, want)
+    assert c != 0 and np.all(np.abs(x / c - want) <= 4 * 2.0 ** -24 * np.abs(want))
