@@ -627,6 +627,34 @@ template <int K> struct EpiZScaleK {
   }
 };
 
+// General M: Z apply and the Richardson step without a weight update (EpiZAxpy, per column)
+template <int K> struct EpiZAxpyK {
+  __half *hout;
+  const RichState *rs;
+  int k;
+  float *out;
+  __half *out16;
+  float isc;
+  float ome[K] = {};  // fp32(ome_c[k]) of every column, set by setup()
+  __device__ __forceinline__ void setup() {
+#pragma unroll
+    for (int c = 0; c < K; c++) ome[c] = h2f(rs[c].ome[k]);
+  }
+  template <typename Acc> __device__ __forceinline__ void row(int64_t r, const Acc (&acc)[K]) const {
+    float h[K], hn[K];
+    RowK<__half, K>::load(hout + r * K, h);
+#pragma unroll
+    for (int c = 0; c < K; c++) hn[c] = h2f(f2h(__fmaf_rn(ome[c], h2f(f2h((float)acc[c])), h[c])));
+    if (out) {
+#pragma unroll
+      for (int c = 0; c < K; c++) hn[c] *= isc;
+      RowK<float, K>::store(out + r * K, hn);
+    } else {
+      RowK<__half, K>::store((out16 ? out16 : hout) + r * K, hn);
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Reductions over K columns.  Two final stages exist, each reproducing one of
 // the single-column kernels' trees exactly:

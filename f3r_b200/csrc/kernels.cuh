@@ -689,6 +689,34 @@ struct EpiZScale {
   template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
 };
 
+// General M, Z apply of a residual step without a weight update, and the step
+// itself: t2 = fp16(Z tmp), hnew = fp16(hout + ome[k] t2) (k_rich_axpy's
+// arithmetic; one pass over t2 and a launch fewer: at 128^3, 7-point, 8.0 us of
+// k_rich_axpy a step), or on the last step out = fp32(hnew) / sc or out16 = hnew.
+struct EpiZAxpy {
+  using Red = float;
+  static constexpr int NV = 0;
+  struct Pre {
+    __half h;
+  };
+  __half *hout;
+  const RichState *rs;
+  int k;
+  float *out;
+  __half *out16;
+  float isc;
+  float ome = 0.0f;  // fp32(ome[k]), set by setup()
+  __device__ __forceinline__ void setup() { ome = h2f(rs->ome[k]); }
+  __device__ __forceinline__ Pre load(int64_t r) const { return {hout[r]}; }
+  template <typename Acc> __device__ __forceinline__ void row(int64_t r, Acc acc, const Pre &p, Red (&)[1]) const {
+    const __half hn = f2h(__fmaf_rn(ome, h2f(f2h((float)acc)), h2f(p.h)));
+    if (out) out[r] = h2f(hn) * isc;
+    else if (out16) out16[r] = hn;
+    else hout[r] = hn;
+  }
+  template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
+};
+
 // fp32 -> fp64 / fp16 / fp32 conversion of a value array (matrix copies).
 template <typename To> __global__ void k_convert_vals(const double *__restrict__ in, To *__restrict__ out, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)

@@ -9,6 +9,7 @@
 
 #include "internal.hpp"
 #include "csr.cuh"
+#include "direct.cuh"
 #include "sell.cuh"
 
 namespace f3r {
@@ -95,6 +96,7 @@ struct DeviceSell {
   int32_t *xoff = nullptr;  // mixed aligned form: per slice, -1 or the explicit indices' offset
   int32_t *rptr = nullptr;  // CSR storage (col = CSR indices, values unpadded), else nullptr
   int32_t height = 32;      // slice height: 32, or 64 (64-row aligned slices)
+  int32_t uw = 0;           // every slice's width where they are all alike, else 0
   uint16_t *dcol = nullptr;
   double *v64 = nullptr;
   float *v32 = nullptr;
@@ -102,7 +104,7 @@ struct DeviceSell {
   int dtypes = 0;
   // 32, 16, or 0 (offset-aligned slices, mixed with explicit ones or not)
   int index_bits() const { return (xoff || (cbase && !dcol)) ? 0 : dcol ? 16 : 32; }
-  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height}; }
+  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, uw}; }
   void release() {
     cudaFree(col); cudaFree(sptr); cudaFree(perm); cudaFree(cbase); cudaFree(cbptr); cudaFree(dcol);
     cudaFree(xoff);
@@ -153,9 +155,37 @@ inline void launch_sell_one(Context &c, const V *val, const DevSell &A, const X 
            sell_smem_bytes<V, CI>(), c.stream, val, A, x, epi, c.err);
 }
 
+template <typename V, typename X, typename Epi, int H, int R>
+inline Status launch_direct_aligned(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
+  launch_k(c, k_sell_direct_aligned<V, X, Epi, H, R>, (unsigned)cdiv(cdiv(A.n, 32 * R) * 32, kDirectThreads),
+           kDirectThreads, 0, c.stream, val, A, x, epi);
+  CUDA_TRY(cudaGetLastError());
+  return F3R_SUCCESS;
+}
+template <typename V, typename X, typename Epi, int UNR>
+inline Status launch_direct_packed(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
+  launch_k(c, k_sell_direct_packed<V, X, Epi, UNR>, (unsigned)cdiv(A.n, kDirectThreads), kDirectThreads, 0, c.stream,
+           val, A, x, epi);
+  CUDA_TRY(cudaGetLastError());
+  return F3R_SUCCESS;
+}
+
 template <typename V, typename X, typename Epi>
 inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
   if (A.nslices == 0) return F3R_SUCCESS;
+  const bool packed = !A.rptr && !A.cbase && !A.xoff && !A.dcol, all_aligned = A.cbase && !A.xoff && !A.dcol;
+  // short rows: thread-a-row kernels (direct.cuh).  Two rows a lane pay off with fp16 values on 64-row
+  // slices (one set of bases) once there is more than one wave of rows: 37.7 -> 33.2 us at 200^3, 1.8 -> 2.1 at 32^3
+  const int64_t wave = (int64_t)c.sm_count * kDirectResident;
+  if (all_aligned && (A.uw == 4 || A.uw == 8)) {
+    if (A.height == 32) return launch_direct_aligned<V, X, Epi, 32, 1>(c, val, A, x, epi);
+    if (sizeof(V) == 2 && A.n > wave) return launch_direct_aligned<V, X, Epi, 64, 2>(c, val, A, x, epi);
+    return launch_direct_aligned<V, X, Epi, 64, 1>(c, val, A, x, epi);
+  }
+  if (packed && A.max_width <= kDirectShort) return launch_direct_packed<V, X, Epi, 4>(c, val, A, x, epi);
+  // small packed matrices: one wave of rows (fp64's take twice the registers: half a wave; at 64^3 the bulk kernel is
+  // ahead there, 15.6 against 16.9 us)
+  if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave)) return launch_direct_packed<V, X, Epi, 8>(c, val, A, x, epi);
   F3R_TRY((sell_attr<V, X, Epi>(c)));
   if (A.height == 64) {
     using C64 = Sell64Cfg<V>;

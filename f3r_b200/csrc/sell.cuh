@@ -67,6 +67,8 @@ struct DevSell {
   int32_t nslices;
   const int32_t *rptr;    // CSR storage: row pointers (col holds the CSR indices), else nullptr
   int32_t height;         // slice height: 32, or 64 (64-row aligned slices, k_sell64)
+  int32_t max_width;      // widest slice
+  int32_t uw;             // the width of every slice where they are all alike (s starts at s * uw), else 0
 };
 
 // Index form of a kernel instantiation.

@@ -348,6 +348,10 @@ Status upload_sell(Context &c, const SellHost &h, int dtype_mask, bool scatter_p
   d.n = h.n; d.ncols = h.ncols; d.nslices = h.nslices; d.max_width = h.max_width; d.sigma = h.sigma;
   d.height = h.height;
   d.nnz = h.nnz; d.nnz_pad = h.nnz_pad; d.dtypes = dtype_mask;
+  // slices of one width (aligned forms: bases from s * width too) need no look-up
+  d.uw = h.nslices > 0 ? h.sptr[1] : 0;
+  for (int32_t s = 0; s < h.nslices && d.uw > 0; s++)
+    if (h.sptr[s + 1] - h.sptr[s] != d.uw || (h.aligned_all && (h.cbptr[s] & ~3) != s * d.uw)) d.uw = 0;
   const size_t np = (size_t)h.nnz_pad;
   if (!h.xoff.empty() || h.aligned_all) {
     const size_t nc = h.cbase.size(), nx = h.col.size();
@@ -750,6 +754,7 @@ template <int K> struct Engine {
       F3R_TRY((launch_block<__half, __half, EpiRichResPreK<K>, K>(C(), h, Av, h, {}, true)));
       F3R_TRY((launch_block<__half, __half, EpiResidualK<__half, __half, K>, K>(C(), h, Av, h, {}, true)));
       F3R_TRY((launch_block<__half, __half, EpiZScaleK<K>, K>(C(), h, Av, h, {}, true)));
+      F3R_TRY((launch_block<__half, __half, EpiZAxpyK<K>, K>(C(), h, Av, h, {}, true)));
       // the Gram-Schmidt update's staging tiles (above 48 KB from K = 16)
       CUDA_TRY(cudaFuncSetAttribute(k_cgs_updateK<float, 8, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)cgs_stage_bytes<float, 8, K>()));
@@ -766,6 +771,7 @@ template <int K> struct Engine {
         F3R_TRY((launch_block_mm<__half, __half, EpiRichResPreK<K, true>, K>(C(), h, Av, h, {}, true)));
         F3R_TRY((launch_block_mm<__half, __half, EpiResidualK<__half, __half, K>, K>(C(), h, Av, h, {}, true)));
         F3R_TRY((launch_block_mm<__half, __half, EpiZScaleK<K>, K>(C(), h, Av, h, {}, true)));
+        F3R_TRY((launch_block_mm<__half, __half, EpiZAxpyK<K>, K>(C(), h, Av, h, {}, true)));
       }
     }
     return F3R_SUCCESS;
@@ -875,6 +881,14 @@ template <int K> struct Engine {
         const bool last = (k == p.m4 - 1);
         F3R_TRY(mv(S.A.v16, Av, (const __half *)w.hout, EpiResidual<__half, __half>{hi, w.hr, nullptr},
                    EpiResidualK<__half, __half, K>{hi, w.hr}));
+        if (!upd && p.precond == F3R_PRECOND_SDAINV) {  // Z's product takes the step with it
+          F3R_TRY(mv_store(S.W.v16, S.W.view(), (const __half *)w.hr, w.tmp));
+          float *fo = last ? out_last : nullptr;
+          __half *ho = last ? out16 : nullptr;
+          F3R_TRY(mv(S.Z.v16, S.Z.view(), (const __half *)w.tmp, EpiZAxpy{w.hout, w.rs, k, fo, ho, isc},
+                     EpiZAxpyK<K>{w.hout, w.rs, k, fo, ho, isc}));
+          continue;
+        }
         F3R_TRY(prec_apply(w.hr, w.tmp2, false));
         if (upd) {
           F3R_TRY(mv_store(S.A.v16, Av, (const __half *)w.tmp2, w.tmp));
@@ -1830,6 +1844,7 @@ static Status make_solver(f3r_context *ctx, const f3r_csr *a, const f3r_params *
   F3R_TRY((sell_attr<__half, __half, EpiStore<float>>(cx)));
   F3R_TRY((sell_attr<float, float, EpiStore<float>>(cx)));
   F3R_TRY((sell_attr<__half, __half, EpiZScale>(cx)));
+  F3R_TRY((sell_attr<__half, __half, EpiZAxpy>(cx)));
   // the single-column workspace (wider ones are made by the first solve_multi that needs them)
   s->z16 = p.m3 > 0 && p.half_scale_log2 == 0 && !(p.inner_sstep & 2) && p.half_m == 0;
   F3R_TRY(make_work<1>(*s, s->w1));
@@ -1871,6 +1886,10 @@ static Status upload_sell_mm(Context &c, const f3r_csr &pattern, const std::vect
     for (int32_t q = 0; q < pattern.nnz; q++) v[(size_t)pos[q] * K + s] = vals[s][q];
   d.n = h.n; d.ncols = h.ncols; d.nslices = h.nslices; d.max_width = h.max_width; d.sigma = 1;
   d.nnz = h.nnz; d.nnz_pad = h.nnz_pad; d.dtypes = dtype_mask;
+  // slices of one width (aligned forms: bases from s * width too) need no look-up
+  d.uw = h.nslices > 0 ? h.sptr[1] : 0;
+  for (int32_t s = 0; s < h.nslices && d.uw > 0; s++)
+    if (h.sptr[s + 1] - h.sptr[s] != d.uw || (h.aligned_all && (h.cbptr[s] & ~3) != s * d.uw)) d.uw = 0;
   F3R_TRY(c.alloc((void **)&d.col, np * 4));
   F3R_TRY(c.alloc((void **)&d.sptr, (size_t)(h.nslices + 1) * 4));
   CUDA_TRY(cudaMemcpyAsync(d.col, h.col.data(), np * 4, cudaMemcpyHostToDevice, c.stream));

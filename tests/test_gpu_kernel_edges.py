@@ -38,3 +38,33 @@ def test_block_ilu_solve_is_the_oracles(ctx, grid, blocks, sigma):
     S.solve(b, x, cond=lambda it, e: it >= 1)
     c = np.dot(x, want) / np.dot(want, want)
     assert c != 0 and np.all(np.abs(x / c - want) <= 4 * 2.0 ** -24 * np.abs(want))
+
+
+@pytest.mark.parametrize("kind,grid,kw", [
+    ("7pt", (64, 3, 2), dict(aligned=True, height=64)), ("7pt", (67, 5, 3), dict(aligned=True)),  # ragged last slices
+    ("7pt", (67, 71, 64), dict(aligned=True, height=64)),  # more than one wave: two rows a lane
+    ("7pt", (67, 71, 64), dict(aligned=True)), ("7pt", (67, 71, 64), dict()),
+    ("7pt", (67, 71, 64), dict(sigma=256)), ("sdainv", (40, 31, 17), dict(aligned=True)),
+    ("27pt", (68, 66, 67), dict()), ("27pt", (70, 68, 66), dict()),  # either side of a wave of rows
+    ("27pt", (53, 53, 53), dict(sigma=256)), ("27pt", (54, 53, 53), dict(sigma=256)),  # and of half of one (fp64)
+])
+def test_thread_a_row_products_bitexact(ctx, kind, grid, kw):
+    """the thread-a-row kernels and the bulk-copy kernels on either side of
+    the rule that chooses between them: the oracle's sums bit for bit"""
+    A = (F.stencil27(*grid, 2, 0.5) if kind == "27pt" else F.diffusion7(*grid, 1.5, 3.0, 1)).scale()
+    if kind == "sdainv":
+        A = A.sdainv()[1]
+    r, i, v = A.arrays()
+    n = A.shape[0]
+    S = F.Sell(ctx, A, **kw)
+    x = np.random.default_rng(1).standard_normal(n)
+    for vt, dt, tdt, ov, oy, oacc in ((F.F64, np.float64, torch.float64, O.DT_F64, O.DT_F64, O.DT_F64),
+                                      (F.F32, np.float32, torch.float32, O.DT_F32, O.DT_F32, O.DT_F32),
+                                      (F.F16, np.float32, torch.float32, O.DT_F16, O.DT_F32, O.DT_F32),
+                                      (F.F16, np.float16, torch.float16, O.DT_F16, O.DT_F16, O.DT_F32)):
+        xd = x.astype(dt)
+        y = torch.zeros(n, dtype=tdt, device="cuda")
+        S.operate(torch.from_numpy(xd).cuda(), y, val_t=vt)
+        torch.cuda.synchronize()
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), O.spmv(r, i, v, xd, ov, oy, oacc).view(np.uint8)), vt
+    S.close()
