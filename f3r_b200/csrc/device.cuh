@@ -38,6 +38,9 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -165,6 +168,12 @@ template <> __device__ __forceinline__ float fma_vx<float, __half, __half>(__hal
   return acc;
 }
 
+
+// fp32 -> fp64 / fp16 / fp32 conversion of a value array (matrix copies).
+template <typename To> __global__ void k_convert_vals(const double *__restrict__ in, To *__restrict__ out, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = cvt<To>(in[i]);
+}
 
 // ---- deterministic grid reduction --------------------------------------------
 // Every block contributes NV partial sums; the last block to arrive adds the

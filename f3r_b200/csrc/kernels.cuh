@@ -583,6 +583,43 @@ template <bool PREFETCH = true, bool UNIT = false> struct EpiRichStepT {
     else hnext[r] = hn;
   }
   template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
+  bool vec4() const {
+    return aligned4(hin) && aligned4(hout) && (out ? aligned4(out) : aligned4(hnext)) && (!M.w || (aligned4(M.w) && aligned4(M.z)));
+  }
+  __device__ __forceinline__ void load4(int64_t r, Pre (&p)[4]) const {
+    __half a[4], b[4];
+    ld4(hin + r, a);
+    ld4(hout + r, b);
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[i].io = __halves2half2(a[i], b[i]);
+    if constexpr (!UNIT) {
+      const VecN<__half, 4> w = M.w4(r), z = M.z4(r);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        p[i].w = w.v[i];
+        p[i].z = z.v[i];
+      }
+    }
+  }
+  template <typename Acc> __device__ __forceinline__ void row4(int64_t r, const Acc (&acc)[4], const Pre (&p)[4],
+                                                                      uint32_t rows) const {
+    __half hn[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const __half hr = f2h(h2f(__low2half(p[i].io)) - (float)acc[i]);
+      __half t2 = hr;
+      if constexpr (!UNIT) t2 = __hmul(p[i].z, __hmul(p[i].w, hr));
+      hn[i] = f2h(__fmaf_rn(ome, h2f(t2), h2f(__high2half(p[i].io))));
+    }
+    if (out) {
+      float o[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) o[i] = h2f(hn[i]) * isc;
+      st4_rows(out + r, o, rows);
+    } else {
+      st4_rows(hnext + r, hn, rows);
+    }
+  }
 };
 using EpiRichStep = EpiRichStepT<true>;
 using EpiRichStepUnit = EpiRichStepT<true, true>;
@@ -716,12 +753,6 @@ struct EpiZAxpy {
   }
   template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
 };
-
-// fp32 -> fp64 / fp16 / fp32 conversion of a value array (matrix copies).
-template <typename To> __global__ void k_convert_vals(const double *__restrict__ in, To *__restrict__ out, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = cvt<To>(in[i]);
-}
 
 // gather / scatter through a row permutation (SELL-C-sigma system order)
 __global__ void k_permute_gather(const double *__restrict__ in, const int32_t *__restrict__ perm,

@@ -10,6 +10,7 @@
 #include "internal.hpp"
 #include "csr.cuh"
 #include "direct.cuh"
+#include "pattern.cuh"
 #include "sell.cuh"
 
 namespace f3r {
@@ -97,6 +98,7 @@ struct DeviceSell {
   int32_t *rptr = nullptr;  // CSR storage (col = CSR indices, values unpadded), else nullptr
   int32_t height = 32;      // slice height: 32, or 64 (64-row aligned slices)
   int32_t uw = 0;           // every slice's width where they are all alike, else 0
+  DevPattern *pat = nullptr;  // the rows' patterns where a few cover the matrix (pattern.cuh)
   uint16_t *dcol = nullptr;
   double *v64 = nullptr;
   float *v32 = nullptr;
@@ -104,11 +106,13 @@ struct DeviceSell {
   int dtypes = 0;
   // 32, 16, or 0 (offset-aligned slices, mixed with explicit ones or not)
   int index_bits() const { return (xoff || (cbase && !dcol)) ? 0 : dcol ? 16 : 32; }
-  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, uw}; }
+  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, uw, pat}; }
   void release() {
     cudaFree(col); cudaFree(sptr); cudaFree(perm); cudaFree(cbase); cudaFree(cbptr); cudaFree(dcol);
     cudaFree(xoff);
     cudaFree(rptr);
+    delete pat;
+    pat = nullptr;
     cbptr = nullptr;
     xoff = nullptr;
     rptr = nullptr;
@@ -142,6 +146,7 @@ inline Status sell_attr(Context &c) {
     using C64 = Sell64Cfg<V>;
     CUDA_TRY(cudaFuncSetAttribute(k_sell64<V, X, Epi, C64::WARPS, C64::STAGES, C64::KC>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sell64_smem_bytes<V>()));
+    CUDA_TRY(cudaFuncSetAttribute(k_sell_pattern<V, X, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     attr_done[c.device & 63] = 1;
   }
   return F3R_SUCCESS;
@@ -170,6 +175,25 @@ inline Status launch_direct_packed(Context &c, const V *val, const DevSell &A, c
   return F3R_SUCCESS;
 }
 
+// false where the windows of x do not fit an SM or x is not on a 16-byte boundary
+template <typename V, typename X, typename Epi>
+inline bool launch_pattern(Context &c, const V *val, const DevPattern &d, const X *x, const Epi &epi) {
+  if (reinterpret_cast<uintptr_t>(x) % 16) return false;
+  const PatShape p = pattern_shape(d.a, d.warps, sizeof(X), sizeof(PatRun<V>));
+  if (p.stages == 0) return false;
+  PatArgs a = d.a;
+  a.stages = p.stages;
+  // the first tile whose windows pass x's last whole 16-byte unit
+  int32_t hi = 0;
+  for (int w = 0; w < a.nwin; w++) hi = std::max(hi, a.win[w].lo + a.win[w].len);
+  const int64_t per = 16 / (int64_t)sizeof(X), nfl = a.n / per * per;
+  a.tail_tile = nfl == a.n ? a.ntiles : (int32_t)std::max<int64_t>(0, (nfl - hi) / a.tile);
+  const int64_t work = std::max<int64_t>(a.ntiles, cdiv(a.ngroups, d.warps));
+  launch_k(c, k_sell_pattern<V, X, Epi>, (unsigned)std::min<int64_t>(work, (int64_t)c.sm_count * p.ctas), (d.warps + 1) * 32,
+           p.smem, c.stream, a, d.tab(val), d.vals(val), x, epi, epi_vec4(epi) ? 1 : 0, c.err);
+  return true;
+}
+
 template <typename V, typename X, typename Epi>
 inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
   if (A.nslices == 0) return F3R_SUCCESS;
@@ -187,6 +211,10 @@ inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x
   // ahead there, 15.6 against 16.9 us)
   if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave)) return launch_direct_packed<V, X, Epi, 8>(c, val, A, x, epi);
   F3R_TRY((sell_attr<V, X, Epi>(c)));
+  if (A.pat && A.n >= pattern_rows(c.sm_count, A.height, sizeof(V)) && launch_pattern(c, val, *A.pat, x, epi)) {
+    CUDA_TRY(cudaGetLastError());
+    return F3R_SUCCESS;
+  }
   if (A.height == 64) {
     using C64 = Sell64Cfg<V>;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(A.nslices, C64::WARPS), c.sm_count));
@@ -236,6 +264,8 @@ double align_offsets(const f3r_csr &a, bool renumber, SellHost &s);
 // every 64-row slice's rows share their column offsets (offset set at most
 // 5/4 of the slice's width), false otherwise (s untouched).
 bool align64(const f3r_csr &a, SellHost &s);
+// The patterns of h's rows, where few enough cover enough of them (pattern.cpp): sets d.pat, or leaves it null.
+Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d);
 // Uploads the value copies selected by dtype_mask (bit 1 << f3r_dtype).
 Status upload_sell(Context &c, const SellHost &h, int dtype_mask, bool scatter_perm, DeviceSell &d);
 // CSR storage with the same value copies (the kernels' CSR path; sigma 1)

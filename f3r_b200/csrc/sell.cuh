@@ -69,6 +69,7 @@ struct DevSell {
   int32_t height;         // slice height: 32, or 64 (64-row aligned slices, k_sell64)
   int32_t max_width;      // widest slice
   int32_t uw;             // the width of every slice where they are all alike (s starts at s * uw), else 0
+  const struct DevPattern *pat;  // host side: the rows' patterns where a few cover the matrix (pattern.cuh), else nullptr
 };
 
 // Index form of a kernel instantiation.
@@ -620,6 +621,34 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 // ---------------------------------------------------------------------------
 struct NoPre {};
 
+// 4 consecutive elements of global memory from a 4-element boundary (of at most 16 bytes)
+template <typename T> __device__ __forceinline__ void ld4(const T *p, T (&o)[4]) {
+  Vec4Load<T>::ld(p, o);
+}
+__device__ __forceinline__ void st4(__half *p, const __half (&v)[4]) {
+  __half2 t[2] = {__halves2half2(v[0], v[1]), __halves2half2(v[2], v[3])};
+  *reinterpret_cast<uint2 *>(p) = *reinterpret_cast<const uint2 *>(t);
+}
+__device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void st4(double *p, const double (&v)[4]) {
+  reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
+  reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
+}
+// the elements of v whose bit is set in rows
+template <typename T> __device__ __forceinline__ void st4_rows(T *p, const T (&v)[4], uint32_t rows) {
+  if (rows == 15u) st4(p, v);
+  else {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if ((rows >> i) & 1u) p[i] = v[i];
+  }
+}
+template <typename T> inline bool aligned4(const T *p) {
+  return reinterpret_cast<uintptr_t>(p) % (sizeof(T) * 4 < 16 ? sizeof(T) * 4 : 16) == 0;
+}
+
 __device__ __forceinline__ int64_t out_row(const int32_t *perm, int64_t r) { return perm ? perm[r] : r; }
 
 // y = A x
@@ -634,6 +663,16 @@ template <typename Out> struct EpiStore {
     y[out_row(perm, r)] = cvt<Out>(acc);
   }
   template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
+  // rows r .. r + 3, r a multiple of 4, in vector accesses where vec4() holds; row4 stores those set in rows
+  bool vec4() const { return !perm && aligned4(y); }
+  __device__ __forceinline__ void load4(int64_t, Pre (&)[4]) const {}
+  template <typename Acc> __device__ __forceinline__ void row4(int64_t r, const Acc (&acc)[4], const Pre (&)[4],
+                                                                      uint32_t rows) const {
+    Out o[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[i] = cvt<Out>(acc[i]);
+    st4_rows(y + r, o, rows);
+  }
 };
 
 // y = b - A x (subtraction in the accumulator type)
@@ -651,6 +690,20 @@ template <typename B, typename Out> struct EpiResidual {
     y[out_row(perm, r)] = cvt<Out>(to_acc<Acc>(p.b) - acc);
   }
   template <int W> __device__ __forceinline__ void finish(Red (&)[1]) const {}
+  bool vec4() const { return !perm && aligned4(y) && aligned4(b); }
+  __device__ __forceinline__ void load4(int64_t r, Pre (&p)[4]) const {
+    B t[4];
+    ld4(b + r, t);
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[i].b = t[i];
+  }
+  template <typename Acc> __device__ __forceinline__ void row4(int64_t r, const Acc (&acc)[4], const Pre (&p)[4],
+                                                                      uint32_t rows) const {
+    Out o[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[i] = cvt<Out>(to_acc<Acc>(p[i].b) - acc[i]);
+    st4_rows(y + r, o, rows);
+  }
 };
 
 }  // namespace f3r

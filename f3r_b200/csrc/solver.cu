@@ -403,7 +403,7 @@ Status upload_sell(Context &c, const SellHost &h, int dtype_mask, bool scatter_p
     cudaFree(tmp64);
   }
   CUDA_TRY(cudaStreamSynchronize(c.stream));
-  return F3R_SUCCESS;
+  return make_pattern(c, h, dtype_mask, d);
 }
 
 // ---------------------------------------------------------------------------

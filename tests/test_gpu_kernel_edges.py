@@ -46,11 +46,15 @@ def test_block_ilu_solve_is_the_oracles(ctx, grid, blocks, sigma):
     ("7pt", (67, 71, 64), dict(aligned=True)), ("7pt", (67, 71, 64), dict()),
     ("7pt", (67, 71, 64), dict(sigma=256)), ("sdainv", (40, 31, 17), dict(aligned=True)),
     ("27pt", (68, 66, 67), dict()), ("27pt", (70, 68, 66), dict()),  # either side of a wave of rows
+    # repeating rows (from half a wave of rows, or a wave): one and three windows, ragged grids, both tile sizes
+    ("27pt", (40, 31, 17), dict(aligned=True, height=64)), ("27pt", (54, 53, 53), dict(aligned=True)),
+    ("27pt", (200, 3, 261), dict(aligned=True)), ("27pt", (101, 67, 59), dict(aligned=True, height=64)),
+    ("27pt", (81, 81, 81), dict(aligned=True)), ("27pt", (97, 90, 81), dict(aligned=True, height=64)),
     ("27pt", (53, 53, 53), dict(sigma=256)), ("27pt", (54, 53, 53), dict(sigma=256)),  # and of half of one (fp64)
 ])
-def test_thread_a_row_products_bitexact(ctx, kind, grid, kw):
-    """the thread-a-row kernels and the bulk-copy kernels on either side of
-    the rule that chooses between them: the oracle's sums bit for bit"""
+def test_products_bitexact_across_the_rules(ctx, kind, grid, kw):
+    """the thread-a-row, the repeating-row and the bulk-copy kernels on either
+    side of the rules that choose between them: the oracle's sums bit for bit"""
     A = (F.stencil27(*grid, 2, 0.5) if kind == "27pt" else F.diffusion7(*grid, 1.5, 3.0, 1)).scale()
     if kind == "sdainv":
         A = A.sdainv()[1]
@@ -66,5 +70,12 @@ def test_thread_a_row_products_bitexact(ctx, kind, grid, kw):
         y = torch.zeros(n, dtype=tdt, device="cuda")
         S.operate(torch.from_numpy(xd).cuda(), y, val_t=vt)
         torch.cuda.synchronize()
-        assert np.array_equal(y.cpu().numpy().view(np.uint8), O.spmv(r, i, v, xd, ov, oy, oacc).view(np.uint8)), vt
+        want = O.spmv(r, i, v, xd, ov, oy, oacc)
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
+        # vectors that start off a 16-byte boundary
+        xo, yo = torch.zeros(n + 1, dtype=tdt, device="cuda")[1:], torch.zeros(n + 1, dtype=tdt, device="cuda")[1:]
+        xo.copy_(torch.from_numpy(xd))
+        S.operate(xo, yo, val_t=vt)
+        torch.cuda.synchronize()
+        assert np.array_equal(yo.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
     S.close()
