@@ -22,7 +22,8 @@
 namespace f3r {
 
 constexpr int kMaxBlock = 16;  // widest block of right-hand sides
-// The single-column (K = 1) BLAS-1 kernels launch 8 blocks of 256 threads per
+// The single-column (K = 1) instances of these BLAS-1 kernels (the fp32 levels
+// of up to 8 steps have their own, blas1.cuh) launch 8 blocks of 256 threads per
 // SM (Context::ew_grid) and declare so (__launch_bounds__(256, 8), at most 32
 // registers a thread), so that the whole grid is resident in one wave.
 
@@ -816,11 +817,10 @@ __global__ void __launch_bounds__(WARPS * 32, K == 1 ? 8 : 1) k_multidot_chunked
 // H(j, k)(c) = <w(:, c), V(k)(:, c)> for nv <= MAXV basis vectors in fp32
 // (k_multidot_f32): rows in groups of 4 per thread, block-strided final stage
 template <int MAXV, int WARPS, int K>
-__global__ void __launch_bounds__(WARPS * 32, K == 1 ? 8 : 1) k_multidot_f32K(const float *__restrict__ w, Cols<float> V, int nv,
+__global__ void __launch_bounds__(WARPS * 32) k_multidot_f32K(const float *__restrict__ w, Cols<float> V, int nv,
                                                               int64_t n, GridRed gr, float *hcol, int64_t hstride) {
-  // basis vectors per pass: single columns take at most 4 (more float4 loads in flight than 32
-  // registers hold spill), K columns up to 32 values
-  constexpr int CV = (MAXV * K > 32) ? (32 / K > 0 ? 32 / K : 1) : (K == 1 && MAXV > 4) ? 4 : MAXV;
+  // basis vectors per pass: up to 32 values (single columns have k_dots1, blas1.cuh)
+  constexpr int CV = MAXV * K > 32 ? (32 / K > 0 ? 32 / K : 1) : MAXV;
   constexpr int NQ = CV * K;
   __shared__ float sred[WARPS][NQ];
   float *part = static_cast<float *>(gr.partials);
@@ -1181,11 +1181,11 @@ __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_zyK(Cols<ZT> Z, 
 }
 
 // First half of R, diagonal M (k_rich_enter_diag), per column: the pending
-// normalisation of in(:, c) (in_inv[c], or none), hin = fp16(in * sc),
+// normalisation of in(:, c) (in_inv[c], or none; written back where store), hin = fp16(in * sc),
 // hout = M hin, times ome_c[0] on a call without a weight update; e_c(0) = 1
 // of the calling level when e_set is given.
 template <bool SCALE_BY_OME, int K, int NR, bool MM>
-__device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ in, bool normalise, const float (&s)[K],
+__device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ in, bool normalise, bool store, const float (&s)[K],
                                                 const float (&om)[K], float sc, const DiagPre &M,
                                                 __half *__restrict__ hin, __half *__restrict__ hout) {
   constexpr int E = NR * K, NM = MM ? E : NR;  // diagonal values: per row, or per row and column
@@ -1195,7 +1195,7 @@ __device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ 
   if (normalise) {
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] *= s[q % K];
-    RowK<float, E>::store(in + i0 * K, v);
+    if (store) RowK<float, E>::store(in + i0 * K, v);
   }
   diag_load<NM>(M.w ? M.w + i0 * (MM ? K : 1) : nullptr, w);
   diag_load<NM>(M.z ? M.z + i0 * (MM ? K : 1) : nullptr, z);
@@ -1214,7 +1214,7 @@ __device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ 
 template <bool SCALE_BY_OME, int K, bool MM = false>
 __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK(float *__restrict__ in, const float *__restrict__ in_inv, float sc, DiagPre M,
                                    __half *__restrict__ hin, __half *__restrict__ hout,
-                                   const RichState *__restrict__ rs, float *e_set, int64_t e_stride, int64_t n) {
+                                   const RichState *__restrict__ rs, float *e_set, int64_t e_stride, int64_t n, bool store) {
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   float om[K], s[K];
 #pragma unroll
@@ -1227,15 +1227,15 @@ __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK
   const int64_t stride = (int64_t)gridDim.x * blockDim.x, tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t ng = n / R;
   for (int64_t q = tid; q < ng; q += stride)
-    rich_enter_rows<SCALE_BY_OME, K, R, MM>(q * R, in, normalise, s, om, sc, M, hin, hout);
+    rich_enter_rows<SCALE_BY_OME, K, R, MM>(q * R, in, normalise, store, s, om, sc, M, hin, hout);
   for (int64_t i = ng * R + tid; i < n; i += stride)
-    rich_enter_rows<SCALE_BY_OME, K, 1, MM>(i, in, normalise, s, om, sc, M, hin, hout);
+    rich_enter_rows<SCALE_BY_OME, K, 1, MM>(i, in, normalise, store, s, om, sc, M, hin, hout);
 }
 
-// General M: (normalise in place), hin = fp16(in * sc) (k_rich_cast_in)
+// General M: (normalise, in place where store), hin = fp16(in * sc) (k_rich_cast_in)
 template <int K>
 __global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict__ in_inv, float sc,
-                                __half *__restrict__ hin, float *e_set, int64_t e_stride, int64_t n) {
+                                __half *__restrict__ hin, float *e_set, int64_t e_stride, int64_t n, bool store) {
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   for_row_groups<RowsPer<K>::R>(n, [&](int64_t i0, auto rows) {
     constexpr int E = decltype(rows)::value * K;
@@ -1244,7 +1244,7 @@ __global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict_
     if (in_inv) {
 #pragma unroll
       for (int q = 0; q < E; q++) v[q] *= in_inv[q % K];
-      RowK<float, E>::store(in + i0 * K, v);
+      if (store) RowK<float, E>::store(in + i0 * K, v);
     }
 #pragma unroll
     for (int q = 0; q < E; q++) h[q] = v[q] * sc;

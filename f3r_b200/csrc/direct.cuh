@@ -132,6 +132,53 @@ __global__ void __launch_bounds__(kDirectThreads)
     if (r0 + 32 * i < A.n) epi.row(r0 + 32 * i, acc[i], pre[i], none);
 }
 
+// Offset-aligned slices that are not all alike: 4 or 8 slots wide (or empty),
+// or with explicit columns among them (the mixed form); a row a lane
+template <typename V, typename X, typename Epi, int H>
+__global__ void __launch_bounds__(kDirectThreads)
+    k_sell_direct_mixed(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+  epi_setup(epi, 0);
+  using Acc = typename acc_of<V>::type;
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= A.n) return;
+  const int32_t s = (int32_t)(r / H), q = (int32_t)(r % H);
+  const int32_t s0 = A.sptr[s], w = A.sptr[s + 1] - s0, cp = A.cbptr[s], xo = A.xoff ? A.xoff[s] : -1;
+  const typename Epi::Pre pre = epi.load(r);
+  const V *lv = val + (size_t)s0 * H + (size_t)q * w;
+  Acc acc = 0;
+  auto row = [&](auto wc) {
+    constexpr int W = decltype(wc)::value;
+    using XB = typename std::conditional<std::is_same<V, __half>::value && std::is_same<X, __half>::value, __half,
+                                         Acc>::type;
+    V v[W];
+    XB xg[W];
+    int32_t c[W];
+    ld_row<V, W>(lv, v);
+    if (xo < 0) {
+#pragma unroll
+      for (int g = 0; g < W / 4; g++) {
+        const int4 b = __ldg(reinterpret_cast<const int4 *>(A.cbase + (cp & ~3)) + g);
+        c[4 * g] = b.x + q; c[4 * g + 1] = b.y + q; c[4 * g + 2] = b.z + q; c[4 * g + 3] = b.w + q;
+      }
+      if (!A.xoff && (cp & 1)) {
+#pragma unroll
+        for (int e = 0; e < W; e++) c[e] = min(max(c[e], 0), A.ncols - 1);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < W; e++) c[e] = __ldg(A.col + (size_t)xo + e * 32 + q);
+    }
+#pragma unroll
+    for (int e = 0; e < W; e++) xg[e] = to_acc<XB>(__ldg(x + c[e]));
+#pragma unroll
+    for (int e = 0; e < W; e++) acc = fma_vx<Acc>(v[e], xg[e], acc);
+  };
+  if (w == 8) row(std::integral_constant<int, 8>());
+  else if (w == 4) row(std::integral_constant<int, 4>());
+  typename Epi::Red none[1];
+  epi.row(r, acc, pre, none);
+}
+
 // Packed int32 slices, UNR columns at a time
 template <typename V, typename X, typename Epi, int UNR>
 __global__ void __launch_bounds__(kDirectThreads)

@@ -167,6 +167,13 @@ inline Status launch_direct_aligned(Context &c, const V *val, const DevSell &A, 
   CUDA_TRY(cudaGetLastError());
   return F3R_SUCCESS;
 }
+template <typename V, typename X, typename Epi, int H>
+inline Status launch_direct_mixed(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
+  launch_k(c, k_sell_direct_mixed<V, X, Epi, H>, (unsigned)cdiv(A.n, kDirectThreads), kDirectThreads, 0, c.stream, val,
+           A, x, epi);
+  CUDA_TRY(cudaGetLastError());
+  return F3R_SUCCESS;
+}
 template <typename V, typename X, typename Epi, int UNR>
 inline Status launch_direct_packed(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
   launch_k(c, k_sell_direct_packed<V, X, Epi, UNR>, (unsigned)cdiv(A.n, kDirectThreads), kDirectThreads, 0, c.stream,
@@ -205,6 +212,10 @@ inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x
     if (A.height == 32) return launch_direct_aligned<V, X, Epi, 32, 1>(c, val, A, x, epi);
     if (sizeof(V) == 2 && A.n > wave) return launch_direct_aligned<V, X, Epi, 64, 2>(c, val, A, x, epi);
     return launch_direct_aligned<V, X, Epi, 64, 1>(c, val, A, x, epi);
+  }
+  if (A.max_width <= kDirectShort && (all_aligned || A.xoff)) {  // mixed form, or slices of 4 and 8 slots
+    if (A.height == 64) return launch_direct_mixed<V, X, Epi, 64>(c, val, A, x, epi);
+    return launch_direct_mixed<V, X, Epi, 32>(c, val, A, x, epi);
   }
   if (packed && A.max_width <= kDirectShort) return launch_direct_packed<V, X, Epi, 4>(c, val, A, x, epi);
   // small packed matrices: one wave of rows (fp64's take twice the registers: half a wave; at 64^3 the bulk kernel is

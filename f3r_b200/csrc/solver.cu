@@ -24,6 +24,7 @@
 #include "internal.hpp"
 #include "kernels.cuh"
 #include "block.cuh"
+#include "blas1.cuh"
 #include "ilu.cuh"
 #include "objects.cuh"
 #include "trsv.hpp"
@@ -556,7 +557,7 @@ template <int K> struct Work {
     F3R_TRY(alloc(&L.sn, (size_t)K * (m + 1)));
     F3R_TRY(alloc(&L.e, (size_t)K * (m + 1)));
     F3R_TRY(alloc(&L.y, (size_t)K * (m + 1)));
-    F3R_TRY(alloc(&L.inv, (size_t)K));
+    F3R_TRY(alloc(&L.inv, (size_t)K * (m + 1)));  // K = 1: one a basis vector (Engine::inv_of), else one a column
     CUDA_TRY(cudaMemsetAsync(L.H, 0, sizeof(T) * (size_t)K * (m + 1) * m, st));
     CUDA_TRY(cudaMemsetAsync(L.e, 0, sizeof(T) * (size_t)K * (m + 1), st));
     return F3R_SUCCESS;
@@ -777,6 +778,26 @@ template <int K> struct Engine {
     return F3R_SUCCESS;
   }
 
+  // Single-column levels of up to kMaxDots1 steps leave their basis vectors
+  // unnormalised and keep every vector's 1/h: R's entry, the dots and the update
+  // multiply it in as they read (blas1.cuh), so no vector is written a second
+  // time.  The fp16-vector and the s-step levels read the stored vectors.
+  bool defer() const {
+    return K == 1 && p.half_m == 0 && p.inner_sstep == 0 && p.m2 >= 1 && p.m2 <= kMaxDots1 && p.m3 <= kMaxDots1;
+  }
+  // where 1/h of basis vector j (j >= 1) is kept
+  template <typename T> T *inv_of(const Level<T> &L, int j) const { return K == 1 ? L.inv + j : L.inv; }
+  // a single-column level's first nv basis vectors with their pending factors;
+  // inv0: that of V(0)
+  Basis8 basis(float *const *Vp, int nv, const Level<float> &L, const float *inv0) const {
+    Basis8 b{};
+    for (int k = 0; k < nv; k++) {
+      b.p[k] = Vp[k];
+      b.s[k] = !defer() ? nullptr : k == 0 ? inv0 : L.inv + k;
+    }
+    return b;
+  }
+
   // ---- outer basis columns, allocated as the solve reaches them ---------------
   Status ensure_outer(int j) {
     while ((int)w.V1.size() < std::min(j + 2, p.m_outer + 1)) {
@@ -834,10 +855,10 @@ template <int K> struct Engine {
         } else {
           if (!upd)
             launch_k(C(), k_rich_enter_diagK<true, 1>, g, kEwThreads, 0, st, in, in_inv, sc, M, w.hin, h0, w.rs, e_set,
-                     e_stride, N);
+                     e_stride, N, !defer());
           else
             launch_k(C(), k_rich_enter_diagK<false, 1>, g, kEwThreads, 0, st, in, in_inv, sc, M, w.hin, h0, w.rs,
-                     e_set, e_stride, N);
+                     e_set, e_stride, N, !defer());
         }
         if (!upd) {
           __half *cur = h0, *nxt = w.hout2;
@@ -870,7 +891,8 @@ template <int K> struct Engine {
       if constexpr (K == 1) {
         if (h16) launch_k(C(), k_rich_cast_in<__half>, g, kEwThreads, 0, st, in16, in_inv, sc, w.hin, e_set, N);
       }
-      if (!h16) launch_k(C(), k_rich_cast_inK<K>, g, kEwThreads, 0, st, in, in_inv, sc, w.hin, e_set, e_stride, N);
+      if (!h16)
+        launch_k(C(), k_rich_cast_inK<K>, g, kEwThreads, 0, st, in, in_inv, sc, w.hin, e_set, e_stride, N, !defer());
       F3R_TRY(prec_apply(hi, h0, !upd));
       if (upd) {
         F3R_TRY(mv_store(S.A.v16, Av, (const __half *)h0, w.tmp));
@@ -916,10 +938,10 @@ template <int K> struct Engine {
     const GridRed gr = w.gr;
     if (!upd)
       launch_k(C(), k_rich_enter_diagK<true, K, MMF>, g, kEwThreads, 0, st, in, in_inv, sc, M, w.hin, h0, w.rs, e_set,
-               e_stride, N);
+               e_stride, N, true);
     else
       launch_k(C(), k_rich_enter_diagK<false, K, MMF>, g, kEwThreads, 0, st, in, in_inv, sc, M, w.hin, h0, w.rs, e_set,
-               e_stride, N);
+               e_stride, N, true);
     if (!upd) {
       __half *cur = h0, *nxt = w.hout2;
       for (int k = 1; k < p.m4; k++) {
@@ -986,26 +1008,57 @@ template <int K> struct Engine {
     return fail(F3R_ERROR_UNSUPPORTED, "block solves take SDAINV only");
   }
 
-  // H(j, 0..nv-1) = <w, V(k)> per column, one pass over w and the basis
-  void dots(const float *wv, const Cols<float> &Vc, int nv, Level<float> &L, int j) {
+  // H(j, 0..nv-1) = <w, V(k)> per column; inv0: V(0)'s pending factor (K = 1)
+  void dots(const float *wv, float *const *Vp, const Cols<float> &Vc, int nv, Level<float> &L, int j, const float *inv0) {
     float *hcol = L.H + (size_t)j * (L.m + 1);
     const int64_t hs = (int64_t)(L.m + 1) * L.m;
-    if (nv <= 4)
-      launch_k(C(), k_multidot_f32K<4, 8, K>, C().ew_grid(cdiv(n, 4)), 256, 0, C().stream, wv, Vc, nv, (int64_t)n,
-               w.gr, hcol, hs);
-    else if (nv <= 8)
-      launch_k(C(), k_multidot_f32K<8, 8, K>, C().ew_grid(cdiv(n, 4)), 256, 0, C().stream, wv, Vc, nv, (int64_t)n,
-               w.gr, hcol, hs);
-    else
-      launch_k(C(), k_multidot_chunkedK<float, 8, K>, C().ew_grid(n), 256, 0, C().stream, wv, Vc, nv, (int64_t)n,
-               w.gr, hcol, hs);
+    const int g4 = C().ew_grid(cdiv(n, 4));
+    if constexpr (K == 1) {
+      if (nv <= kMaxDots1) {
+        // two logical blocks a block once the grid passes the residency of 4 blocks an SM
+        const Basis8 b = basis(Vp, nv, L, inv0);
+        const bool two = g4 > 4 * C().sm_count;
+        const int g = two ? (int)cdiv(g4, 2) : g4;
+        auto go = [&](auto k) { launch_k(C(), k, g, 256, 0, C().stream, wv, b, nv, (int64_t)n, g4, w.gr, hcol); };
+        if (nv <= 4) two ? go(k_dots1<4, 2>) : go(k_dots1<4, 1>);
+        else two ? go(k_dots1<8, 2>) : go(k_dots1<8, 1>);
+        return;
+      }
+    } else {
+      if (nv <= 4) {
+        launch_k(C(), k_multidot_f32K<4, 8, K>, g4, 256, 0, C().stream, wv, Vc, nv, (int64_t)n, w.gr, hcol, hs);
+        return;
+      }
+      if (nv <= 8) {
+        launch_k(C(), k_multidot_f32K<8, 8, K>, g4, 256, 0, C().stream, wv, Vc, nv, (int64_t)n, w.gr, hcol, hs);
+        return;
+      }
+    }
+    launch_k(C(), k_multidot_chunkedK<float, 8, K>, C().ew_grid(n), 256, 0, C().stream, wv, Vc, nv, (int64_t)n,
+             w.gr, hcol, hs);
   }
 
   // the Gram-Schmidt update, norm and Givens of step j of an inner level
-  void cgs(float *wv, const Cols<float> &Vc, int nv, Level<float> &L, int j, bool last) {
-    launch_k(C(), k_cgs_updateK<float, 8, K>, C().ew_grid(cdiv(n, 4)), 256, cgs_stage_bytes<float, 8, K>(),
-             C().stream, wv, Vc, nv, (int64_t)n, w.gr, L.view(), j, last ? 1 : 0, (double *)nullptr,
-             (const uint32_t *)w.active, C().err);
+  void cgs(float *wv, float *const *Vp, const Cols<float> &Vc, int nv, Level<float> &L, int j, bool last,
+           const float *inv0) {
+    const int g4 = C().ew_grid(cdiv(n, 4));
+    LevelK<float> Lv = L.view();
+    if constexpr (K == 1) {
+      Lv.inv = inv_of(L, j + 1);
+      if (nv <= kMaxDots1) {
+        const Basis8 b = basis(Vp, nv, L, inv0);
+        const bool two = g4 > 4 * C().sm_count;
+        const int g = two ? (int)cdiv(g4, 2) : g4;
+        auto go = [&](auto k) {
+          launch_k(C(), k, g, 256, 0, C().stream, wv, b, nv, (int64_t)n, g4, w.gr, Lv, j, last ? 1 : 0, C().err);
+        };
+        if (nv <= 4) two ? go(k_cgs1<4, 2>) : go(k_cgs1<4, 1>);
+        else two ? go(k_cgs1<8, 2>) : go(k_cgs1<8, 1>);
+        return;
+      }
+    }
+    launch_k(C(), k_cgs_updateK<float, 8, K>, g4, 256, cgs_stage_bytes<float, 8, K>(), C().stream, wv, Vc, nv,
+             (int64_t)n, w.gr, Lv, j, last ? 1 : 0, (double *)nullptr, (const uint32_t *)w.active, C().err);
   }
 
   // sFGMRES's second and third loops (gmres2.hpp:181-193), K = 1: classical
@@ -1017,10 +1070,11 @@ template <int K> struct Engine {
     const int64_t N = n;
     for (int j = 0; j < L.m; j++) {
       float *wv = Vp[j + 1];
-      dots(wv, V, j + 1, L, j);
-      cgs(wv, V, j + 1, L, j, j == L.m - 1);
+      dots(wv, Vp, V, j + 1, L, j, nullptr);
+      cgs(wv, Vp, V, j + 1, L, j, j == L.m - 1, nullptr);
       if (j + 1 < L.m)
-        launch_k(C(), k_scale<float>, C().ew_grid(cdiv(N, 4)), kEwThreads, 0, C().stream, wv, (const float *)L.inv, N);
+        launch_k(C(), k_scale<float>, C().ew_grid(cdiv(N, 4)), kEwThreads, 0, C().stream, wv,
+                 (const float *)inv_of(L, j + 1), N);
     }
     CUDA_TRY(cudaGetLastError());
     return F3R_SUCCESS;
@@ -1081,9 +1135,10 @@ template <int K> struct Engine {
 
   // ---- level 3: FGMRES<float>(A16, R, m3), input a level-2 block column, output
   // a level-2 Z column.  The normalisation V(j+1) *= 1/h of every basis vector
-  // is deferred to the first kernel that reads it next (R's entry), which
-  // scales it in place; the last basis vector of a level is never read again
-  // and is left unscaled.  in_inv: the pending factors of `in` (nullptr if none).
+  // is deferred to the kernels that read it: all of them where defer() holds,
+  // else the first one (R's entry), which scales it in place; the last basis
+  // vector of a level is never read again and is left unscaled.  in_inv: the
+  // pending factors of `in` (nullptr if none).
   Status level3(float *in, float *out, const float *in_inv) {
     Level<float> &L = w.L3;
     float *Vp[kMaxCols];
@@ -1109,10 +1164,18 @@ template <int K> struct Engine {
         for (int j = 0; j < L.m; j++) {
           __half *zj = w.Z16 + (size_t)j * lk();
           float *wv = Vp[j + 1];
-          F3R_TRY(inner_apply(Vp[j], nullptr, j == 0 ? L.e : nullptr, es, j == 0 ? in_inv : L.inv, zj));
+          F3R_TRY(inner_apply(Vp[j], nullptr, j == 0 ? L.e : nullptr, es, j == 0 ? in_inv : inv_of(L, j), zj));
           F3R_TRY(mv_store(S.A.v16, S.A.view(), (const __half *)zj, wv));
-          dots(wv, V, j + 1, L, j);
-          cgs(wv, V, j + 1, L, j, j == L.m - 1);
+          dots(wv, Vp, V, j + 1, L, j, in_inv);
+          cgs(wv, Vp, V, j + 1, L, j, j == L.m - 1, in_inv);
+        }
+        if constexpr (K == 1) {
+          if (L.m <= kMaxDots1) {
+            launch_k(C(), k_zy1, (unsigned)cdiv(n, 2048), 256, 0, C().stream, (const __half *)w.Z16, lk(),
+                     (const float *)L.y, L.m, out, (int64_t)n);
+            CUDA_TRY(cudaGetLastError());
+            return F3R_SUCCESS;
+          }
         }
         launch_k(C(), k_zyK<float, float, false, K, __half>, C().ew_grid(n), kEwThreads, 0, C().stream, Z16,
                  (const float *)L.y, (int64_t)(L.m + 1), L.m, out, (float *const *)nullptr, 0u, (int64_t)n);
@@ -1123,10 +1186,10 @@ template <int K> struct Engine {
       for (int j = 0; j < L.m; j++) {
         float *zj = L.Z + (size_t)j * lk();
         float *wv = Vp[j + 1];
-        F3R_TRY(inner_apply(Vp[j], zj, j == 0 ? L.e : nullptr, es, j == 0 ? in_inv : L.inv));
+        F3R_TRY(inner_apply(Vp[j], zj, j == 0 ? L.e : nullptr, es, j == 0 ? in_inv : inv_of(L, j)));
         F3R_TRY(mv_store(S.A.v16, S.A.view(), (const float *)zj, wv));
-        dots(wv, V, j + 1, L, j);
-        cgs(wv, V, j + 1, L, j, j == L.m - 1);
+        dots(wv, Vp, V, j + 1, L, j, in_inv);
+        cgs(wv, Vp, V, j + 1, L, j, j == L.m - 1, in_inv);
       }
     }
     launch_k(C(), k_zyK<float, float, false, K>, C().ew_grid(n), kEwThreads, 0, C().stream, Zc, (const float *)L.y,
@@ -1158,11 +1221,11 @@ template <int K> struct Engine {
       for (int j = 0; j < L.m; j++) {
         float *zj = L.Z + (size_t)j * lk();
         float *wv = Vp[j + 1];
-        if (p.m3 > 0) F3R_TRY(level3(Vp[j], zj, j == 0 ? nullptr : L.inv));
-        else F3R_TRY(inner_apply(Vp[j], zj, nullptr, 0, j == 0 ? nullptr : L.inv));  // depth 2: R directly
+        if (p.m3 > 0) F3R_TRY(level3(Vp[j], zj, j == 0 ? nullptr : inv_of(L, j)));
+        else F3R_TRY(inner_apply(Vp[j], zj, nullptr, 0, j == 0 ? nullptr : inv_of(L, j)));  // depth 2: R directly
         F3R_TRY(mv_store(S.A.v32, S.A.view(), (const float *)zj, wv));
-        dots(wv, V, j + 1, L, j);
-        cgs(wv, V, j + 1, L, j, j == L.m - 1);
+        dots(wv, Vp, V, j + 1, L, j, nullptr);
+        cgs(wv, Vp, V, j + 1, L, j, j == L.m - 1, nullptr);
       }
     }
     launch_k(C(), k_zyK<float, double, false, K>, C().ew_grid(n), kEwThreads, 0, C().stream, Zc, (const float *)L.y,

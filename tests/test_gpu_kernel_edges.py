@@ -79,3 +79,22 @@ def test_products_bitexact_across_the_rules(ctx, kind, grid, kw):
         torch.cuda.synchronize()
         assert np.array_equal(yo.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
     S.close()
+
+
+@pytest.mark.parametrize("grid", [(13, 11, 7), (32, 32, 32), (70, 69, 63), (97, 90, 71)])
+@pytest.mark.parametrize("m2,m3", [(8, 4), (3, 8), (5, 0)])
+def test_single_column_levels_are_the_block_kernels(ctx, grid, m2, m3):
+    """the single solve's dots, updates and deferred normalisation against the
+    K-column kernels: a column of a two-column block, bit for bit, with one and
+    two logical blocks a block, 1 to 8 basis vectors and n % 4 of 0 to 3"""
+    A = F.stencil27(*grid, 2, 0.5).scale()
+    n = A.shape[0]
+    X = np.stack([F.random_uniform(k, -1.0, 1.0, n) for k in (1, 2)])
+    B = np.stack([A.spmv(x) for x in X])
+    S = F.Solver(ctx, A, rel_tol=1e-10, m2=m2, m3=m3, sell_align=1)
+    Y = np.zeros_like(B)
+    rb = S.solve_multi(B, Y)
+    for k in (0, 1):
+        y = np.zeros(n)
+        r = S.solve(B[k], y)
+        assert r.is_solved and r.res_iter == rb[k].res_iter and np.array_equal(y, Y[k])
