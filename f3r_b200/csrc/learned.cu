@@ -17,15 +17,16 @@
 // should map a residual to its error.  Several systems of one grid shape are
 // trained together as one block-diagonal system.  Kernels (fp32 master
 // weights, fp64 sparse products):
-//   forward    one thread per row, the weights in shared memory
+//   forward    persistent blocks of 128 threads over tiles of 128 rows, register-
+//              tiled layers (8 rows x 8 units a thread), weights in shared memory
 //   pairs      u = W'^T r, y = Z' u, d = dL/dy, g = Z'^T d over all pairs
 //              (blockIdx.y = pair); entry gradients dZ'_ij = sum_p d_i u_j and
 //              dW'^T_jk = sum_p g_j r_k, folded into per-row output gradients
 //              dO[row][slot] = dv' * v
-//   backward   persistent blocks of 128 threads, one row each: the block
-//              recomputes its tile's activations into shared memory, forms the
-//              weight gradients as sums over the tile's rows into a shared
-//              accumulator, and adds that to the global gradient once
+//   backward   the same blocks: a block recomputes its tile's activations into
+//              shared memory, forms the weight gradients as sums over the
+//              tile's rows, keeps their totals in registers, and adds those to
+//              the global gradient once
 //   Adam       one thread per parameter
 // Inference runs the same network in BF16 on the tensor cores with fp32
 // accumulation: tcgen05.mma with TMEM accumulators, one warpgroup per 128-row
@@ -50,11 +51,13 @@ constexpr int kH = 64;     // hidden width
 constexpr int kIn = 7;     // coefficients per row
 constexpr int kOut = 8;    // Z slots 0..3, W^T slots 4..7
 constexpr int kRows = 128; // rows per tile in the training kernels
-constexpr int kLdH = kH + 1, kLdO = kOut + 1;  // padded shared-memory rows (no bank conflicts)
+constexpr int kPitch = kRows + 4;  // a unit's values over the tile's rows in shared memory (16-byte steps free of bank conflicts)
 // flat parameter layout: W1 (kH x kIn), b1, W2 (kH x kH), b2, W3 (kOut x kH), b3; W row-major (out x in)
 constexpr int oW1 = 0, oB1 = oW1 + kH * kIn, oW2 = oB1 + kH, oB2 = oW2 + kH * kH, oW3 = oB2 + kH,
               oB3 = oW3 + kOut * kH, kParams = oB3 + kOut;
-constexpr size_t kBackSmem = sizeof(float) * (2 * kParams + 2 * kRows * kLdH + kRows * kLdO);
+constexpr size_t kForwardSmem = sizeof(float) * (kParams + (8 + 2 * kH) * kPitch);
+constexpr size_t kBackSmem = sizeof(float) * (kParams + (16 + 2 * kH) * kPitch);
+static_assert(kParams % 4 == 0 && oW2 % 4 == 0 && oW3 % 4 == 0, "16-byte rows of the weights");
 
 // One (possibly block-diagonal) system on the device: A, the factors with the
 // slot of every entry, Z's transposed pattern, features, outputs, and the
@@ -109,40 +112,127 @@ __global__ void k_features(int32_t n, int32_t nx, int32_t sxy, const int32_t *__
   for (int s = 0; s < kIn; s++) f[i * kIn + s] = o[s];
 }
 
-__device__ __forceinline__ void load_params(float *sp, const float *__restrict__ p) {
-  for (int k = threadIdx.x; k < kParams; k += blockDim.x) sp[k] = p[k];
+// ---- fp32 network over tiles of kRows rows, kRows threads -------------------
+// Activations lie unit by unit in shared memory (value of unit k, row r at
+// k * kPitch + r).  The two 64 x 64 layers, forward and backward, and the
+// weight gradients are register-tiled products: a thread holds 8 rows x 8 units
+// (or 8 x 4 weights) and takes 16-byte loads, 11 to 16 multiply-adds for each;
+// one row a thread took one or two loads for every multiply-add.  Sums run in
+// the order of the scalar loops: bias first, then the inputs in order; a tile's
+// rows in order, then tile by tile.  Bound by FMA issue (two CTAs an SM).
+// 221,184 rows: forward 138 -> 63 us, backward 684 -> 179 us.
+struct MlpThread {
+  int rt, ut;  // rows 4 rt + {0..3} and 64 + 4 rt + {0..3}; units 8 ut + {0..7}
+  __device__ __forceinline__ MlpThread() : rt(threadIdx.x % 16), ut(threadIdx.x / 16) {}
+  __device__ __forceinline__ void load(const float *unit, float (&o)[8]) const {
+    const float4 a = *reinterpret_cast<const float4 *>(unit + 4 * rt);
+    const float4 b = *reinterpret_cast<const float4 *>(unit + 64 + 4 * rt);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+  }
+  __device__ __forceinline__ void store(float *unit, const float (&v)[8]) const {
+    *reinterpret_cast<float4 *>(unit + 4 * rt) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4 *>(unit + 64 + 4 * rt) = make_float4(v[4], v[5], v[6], v[7]);
+  }
+};
+
+// features of the tile (thread = row): XT, with ones in unit 7 for the rows that exist
+__device__ __forceinline__ void mlp_features(const float *__restrict__ f, int64_t i, bool live, float *XT) {
+#pragma unroll
+  for (int c = 0; c < kIn; c++) XT[c * kPitch + threadIdx.x] = live ? f[i * kIn + c] : 0.f;
+  XT[kIn * kPitch + threadIdx.x] = live ? 1.f : 0.f;
+}
+
+// H1 = relu(W1 X + b1), then H2 = relu(W2 H1 + b2) of the tile; ends with a barrier
+__device__ __forceinline__ void mlp_hidden(const float *sp, const float *XT, float *H1, float *H2) {
+  const MlpThread t;
+  float acc[8][8];  // [unit][row]
+#pragma unroll
+  for (int u = 0; u < 8; u++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[u][r] = sp[oB1 + 8 * t.ut + u];
+#pragma unroll
+  for (int c = 0; c < kIn; c++) {
+    float x[8];
+    t.load(XT + c * kPitch, x);
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const float w = sp[oW1 + (8 * t.ut + u) * kIn + c];
+#pragma unroll
+      for (int r = 0; r < 8; r++) acc[u][r] = fmaf(w, x[r], acc[u][r]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[u][r] = relu(acc[u][r]);
+    t.store(H1 + (8 * t.ut + u) * kPitch, acc[u]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; u++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[u][r] = sp[oB2 + 8 * t.ut + u];
+#pragma unroll 2
+  for (int k0 = 0; k0 < kH; k0 += 4) {
+    float h[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) t.load(H1 + (k0 + k) * kPitch, h[k]);
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const float4 w = *reinterpret_cast<const float4 *>(sp + oW2 + (8 * t.ut + u) * kH + k0);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        acc[u][r] = fmaf(w.x, h[0][r], acc[u][r]);
+        acc[u][r] = fmaf(w.y, h[1][r], acc[u][r]);
+        acc[u][r] = fmaf(w.z, h[2][r], acc[u][r]);
+        acc[u][r] = fmaf(w.w, h[3][r], acc[u][r]);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[u][r] = relu(acc[u][r]);
+    t.store(H2 + (8 * t.ut + u) * kPitch, acc[u]);
+  }
   __syncthreads();
 }
 
-// o = W3 relu(W2 relu(W1 f + b1) + b2) + b3, one thread per row (fp32)
-__global__ void __launch_bounds__(kRows) k_mlp_forward(int32_t n, const float *__restrict__ f,
-                                                      const float *__restrict__ p, float *__restrict__ o) {
-  __shared__ float sp[kParams];
-  load_params(sp, p);
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float x[kIn], h1[kH], acc[kOut];
+// o = W3 relu(W2 relu(W1 f + b1) + b2) + b3 (fp32); persistent blocks
+__global__ void __launch_bounds__(kRows, 2) k_mlp_forward(int32_t n, const float *__restrict__ f,
+                                                         const float *__restrict__ p, float *__restrict__ o) {
+  extern __shared__ __align__(16) float sm[];
+  float *sp = sm, *XT = sp + kParams, *H1 = XT + 8 * kPitch, *H2 = H1 + kH * kPitch;
+  for (int k = threadIdx.x; k < kParams; k += kRows) sp[k] = p[k];
+  const int64_t ntiles = (n + kRows - 1) / kRows;
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int64_t i = tile * kRows + threadIdx.x;
+    mlp_features(f, i, i < n, XT);
+    __syncthreads();
+    mlp_hidden(sp, XT, H1, H2);
+    float acc[kOut];
 #pragma unroll
-  for (int c = 0; c < kIn; c++) x[c] = f[i * kIn + c];
+    for (int s = 0; s < kOut; s++) acc[s] = sp[oB3 + s];
+#pragma unroll 4
+    for (int k0 = 0; k0 < kH; k0 += 4) {
+      float h[4];
 #pragma unroll
-  for (int j = 0; j < kH; j++) {
-    float s = sp[oB1 + j];
+      for (int k = 0; k < 4; k++) h[k] = H2[(k0 + k) * kPitch + threadIdx.x];
 #pragma unroll
-    for (int c = 0; c < kIn; c++) s = fmaf(sp[oW1 + j * kIn + c], x[c], s);
-    h1[j] = relu(s);
+      for (int s = 0; s < kOut; s++) {
+        const float4 w = *reinterpret_cast<const float4 *>(sp + oW3 + s * kH + k0);
+        acc[s] = fmaf(w.x, h[0], acc[s]);
+        acc[s] = fmaf(w.y, h[1], acc[s]);
+        acc[s] = fmaf(w.z, h[2], acc[s]);
+        acc[s] = fmaf(w.w, h[3], acc[s]);
+      }
+    }
+    if (i < n) {
+      reinterpret_cast<float4 *>(o + i * kOut)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      reinterpret_cast<float4 *>(o + i * kOut)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
   }
-#pragma unroll
-  for (int t = 0; t < kOut; t++) acc[t] = sp[oB3 + t];
-  for (int k = 0; k < kH; k++) {
-    float s = sp[oB2 + k];
-#pragma unroll
-    for (int j = 0; j < kH; j++) s = fmaf(sp[oW2 + k * kH + j], h1[j], s);
-    const float h2 = relu(s);
-#pragma unroll
-    for (int t = 0; t < kOut; t++) acc[t] = fmaf(sp[oW3 + t * kH + k], h2, acc[t]);
-  }
-#pragma unroll
-  for (int t = 0; t < kOut; t++) o[i * kOut + t] = acc[t];
 }
 
 // v' = v (1 + delta[row][slot0 + slot]) for every entry with a slot
@@ -236,106 +326,175 @@ __global__ void k_entry_grad(int32_t n, int32_t npairs, const int32_t *__restric
   for (int k = 0; k < kOut; k++) dout[i * kOut + k] = (float)acc[k];
 }
 
-// Backward through the MLP.  Persistent blocks of kRows threads walk tiles of
-// kRows rows (thread t = row t of the tile); rows past n contribute zeros.
-// Shared memory: the parameters, their gradient accumulator, H1 / H2 (the
-// activations, overwritten by the pre-activation gradients) and dO.
-__global__ void __launch_bounds__(kRows) k_mlp_backward(int32_t n, const float *__restrict__ f,
-                                                       const float *__restrict__ p,
-                                                       const float *__restrict__ dout, float *__restrict__ grad) {
-  extern __shared__ float sm[];
-  float *sp = sm;                   // kParams
-  float *G = sp + kParams;          // kParams (gradient accumulator)
-  float *H1 = G + kParams;          // kRows x kLdH
-  float *H2 = H1 + kRows * kLdH;    // kRows x kLdH
-  float *DO = H2 + kRows * kLdH;    // kRows x kLdO
-  for (int k = threadIdx.x; k < kParams; k += blockDim.x) {
-    sp[k] = p[k];
-    G[k] = 0.f;
+// sum over the tile's rows, in order, of a[r] b[r] onto s
+__device__ __forceinline__ float mlp_dot4(const float4 a, const float4 b, float s) {
+  s = fmaf(a.x, b.x, s);
+  s = fmaf(a.y, b.y, s);
+  s = fmaf(a.z, b.z, s);
+  return fmaf(a.w, b.w, s);
+}
+
+// Backward through the MLP, persistent blocks over tiles of kRows rows; rows
+// past n contribute zeros.  A block recomputes its tile's activations, and every
+// thread keeps the totals of its weights over the block's tiles in registers:
+// dW2 (8 ut + a, rt + 16 b), dW3 (ut, rt + 16 b) and dW1 (rt + 16 b, ut; the
+// eighth feature of ones gives db1), db2 on threads 0..63, db3 on 64..71.
+__global__ void __launch_bounds__(kRows, 2) k_mlp_backward(int32_t n, const float *__restrict__ f,
+                                                          const float *__restrict__ p,
+                                                          const float *__restrict__ dout, float *__restrict__ grad) {
+  extern __shared__ __align__(16) float sm[];
+  float *sp = sm, *XT = sp + kParams, *DO = XT + 8 * kPitch, *H1 = DO + 8 * kPitch, *H2 = H1 + kH * kPitch;
+  const int tid = threadIdx.x;
+  const MlpThread t;
+  for (int k = tid; k < kParams; k += kRows) sp[k] = p[k];
+  float g2[8][4], g3[4], g1[4], gb = 0.f;
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    g3[b] = g1[b] = 0.f;
+#pragma unroll
+    for (int a = 0; a < 8; a++) g2[a][b] = 0.f;
   }
-  __syncthreads();
-  const int t = threadIdx.x;
+  auto quad = [](const float *q, int r) { return *reinterpret_cast<const float4 *>(q + r); };
   const int64_t ntiles = (n + kRows - 1) / kRows;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t row0 = tile * kRows, i = row0 + t;
+    const int64_t i = tile * kRows + tid;
     const bool live = i < n;
-    float x[kIn];
+    mlp_features(f, i, live, XT);
 #pragma unroll
-    for (int c = 0; c < kIn; c++) x[c] = live ? f[i * kIn + c] : 0.f;
-    for (int j = 0; j < kH; j++) {
-      float s = sp[oB1 + j];
-#pragma unroll
-      for (int c = 0; c < kIn; c++) s = fmaf(sp[oW1 + j * kIn + c], x[c], s);
-      H1[t * kLdH + j] = live ? relu(s) : 0.f;
-    }
-    for (int k = 0; k < kH; k++) {
-      float s = sp[oB2 + k];
-      for (int j = 0; j < kH; j++) s = fmaf(sp[oW2 + k * kH + j], H1[t * kLdH + j], s);
-      H2[t * kLdH + k] = live ? relu(s) : 0.f;
-    }
-#pragma unroll
-    for (int s = 0; s < kOut; s++) DO[t * kLdO + s] = live ? dout[i * kOut + s] : 0.f;
+    for (int s = 0; s < kOut; s++) DO[s * kPitch + tid] = live ? dout[i * kOut + s] : 0.f;
     __syncthreads();
-    // dW3 (kOut x kH) and db3 over the tile's rows
-    for (int q = t; q < kOut * kH + kOut; q += kRows) {
-      float s = 0;
-      if (q < kOut * kH) {
-        const int so = q / kH, k = q % kH;
-        for (int rr = 0; rr < kRows; rr++) s = fmaf(DO[rr * kLdO + so], H2[rr * kLdH + k], s);
-        G[oW3 + q] += s;
-      } else {
-        const int so = q - kOut * kH;
-        for (int rr = 0; rr < kRows; rr++) s += DO[rr * kLdO + so];
-        G[oB3 + so] += s;
+    mlp_hidden(sp, XT, H1, H2);
+    // dW3 (kOut x kH), db3
+    {
+      float s3[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int r = 0; r < kRows; r += 4) {
+        const float4 d = quad(DO + t.ut * kPitch, r);
+#pragma unroll
+        for (int b = 0; b < 4; b++) s3[b] = mlp_dot4(d, quad(H2 + (t.rt + 16 * b) * kPitch, r), s3[b]);
+      }
+#pragma unroll
+      for (int b = 0; b < 4; b++) g3[b] += s3[b];
+    }
+    __syncthreads();
+    // dh2pre = (W3^T dO) [h2 > 0], in place of h2 (own rows and units only)
+    {
+      float d[8][8];  // [unit][row]
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) d[u][r] = 0.f;
+#pragma unroll
+      for (int s = 0; s < kOut; s++) {
+        float x[8];
+        t.load(DO + s * kPitch, x);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const float w = sp[oW3 + s * kH + 8 * t.ut + u];
+#pragma unroll
+          for (int r = 0; r < 8; r++) d[u][r] = fmaf(w, x[r], d[u][r]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        float h[8];
+        t.load(H2 + (8 * t.ut + u) * kPitch, h);
+#pragma unroll
+        for (int r = 0; r < 8; r++) d[u][r] = h[r] > 0.f ? d[u][r] : 0.f;
+        t.store(H2 + (8 * t.ut + u) * kPitch, d[u]);
       }
     }
     __syncthreads();
-    // dh2pre = (W3^T dO) [h2 > 0], in place of h2 (own row only)
-    for (int k = 0; k < kH; k++) {
-      float s = 0;
+    // dW2 (kH x kH) = dH2pre^T H1
+    {
+      float s2[8][4];
 #pragma unroll
-      for (int so = 0; so < kOut; so++) s = fmaf(sp[oW3 + so * kH + k], DO[t * kLdO + so], s);
-      H2[t * kLdH + k] = H2[t * kLdH + k] > 0.f ? s : 0.f;
+      for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) s2[a][b] = 0.f;
+      for (int r = 0; r < kRows; r += 4) {
+        float4 h[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) h[b] = quad(H1 + (t.rt + 16 * b) * kPitch, r);
+#pragma unroll
+        for (int a = 0; a < 8; a++) {
+          const float4 d = quad(H2 + (8 * t.ut + a) * kPitch, r);
+#pragma unroll
+          for (int b = 0; b < 4; b++) s2[a][b] = mlp_dot4(d, h[b], s2[a][b]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) g2[a][b] += s2[a][b];
     }
-    __syncthreads();
-    // dW2 (kH x kH) = dH2pre^T H1, db2
-    for (int q = t; q < kH * kH + kH; q += kRows) {
-      float s = 0;
-      if (q < kH * kH) {
-        const int k = q / kH, j = q % kH;
-        for (int rr = 0; rr < kRows; rr++) s = fmaf(H2[rr * kLdH + k], H1[rr * kLdH + j], s);
-        G[oW2 + q] += s;
-      } else {
-        const int k = q - kH * kH;
-        for (int rr = 0; rr < kRows; rr++) s += H2[rr * kLdH + k];
-        G[oB2 + k] += s;
+    // db2, db3
+    if (tid < kH + kOut) {
+      const float *q = tid < kH ? H2 + tid * kPitch : DO + (tid - kH) * kPitch;
+      float s = 0.f;
+#pragma unroll 4
+      for (int r = 0; r < kRows; r += 4) {
+        const float4 d = quad(q, r);
+        s += d.x;
+        s += d.y;
+        s += d.z;
+        s += d.w;
+      }
+      gb += s;
+    }
+    // dh1pre = (W2^T dh2pre) [h1 > 0], in place of h1
+    {
+      float d[8][8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) d[u][r] = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < kH; k++) {
+        float x[8];
+        t.load(H2 + k * kPitch, x);
+        const float4 w0 = quad(sp + oW2 + k * kH + 8 * t.ut, 0), w1 = quad(sp + oW2 + k * kH + 8 * t.ut, 4);
+        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+#pragma unroll
+          for (int r = 0; r < 8; r++) d[u][r] = fmaf(w[u], x[r], d[u][r]);
+      }
+      __syncthreads();  // every thread is past its reads of h1
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        float h[8];
+        t.load(H1 + (8 * t.ut + u) * kPitch, h);
+#pragma unroll
+        for (int r = 0; r < 8; r++) d[u][r] = h[r] > 0.f ? d[u][r] : 0.f;
+        t.store(H1 + (8 * t.ut + u) * kPitch, d[u]);
       }
     }
     __syncthreads();
-    // dh1pre = (W2^T dh2pre) [h1 > 0], in place of h1 (own row only)
-    for (int j = 0; j < kH; j++) {
-      float s = 0;
-      for (int k = 0; k < kH; k++) s = fmaf(sp[oW2 + k * kH + j], H2[t * kLdH + k], s);
-      H1[t * kLdH + j] = H1[t * kLdH + j] > 0.f ? s : 0.f;
-    }
-    __syncthreads();
-    // dW1 (kH x kIn) = dH1pre^T X, db1 (X read again from global memory)
-    for (int q = t; q < kH * kIn + kH; q += kRows) {
-      float s = 0;
-      if (q < kH * kIn) {
-        const int j = q / kIn, c = q % kIn;
-        for (int rr = 0; rr < kRows; rr++)
-          if (row0 + rr < n) s = fmaf(H1[rr * kLdH + j], f[(row0 + rr) * kIn + c], s);
-        G[oW1 + q] += s;
-      } else {
-        const int j = q - kH * kIn;
-        for (int rr = 0; rr < kRows; rr++) s += H1[rr * kLdH + j];
-        G[oB1 + j] += s;
+    // dW1 (kH x kIn) and db1 = dH1pre^T (X, 1)
+    {
+      float s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int r = 0; r < kRows; r += 4) {
+        const float4 x = quad(XT + t.ut * kPitch, r);
+#pragma unroll
+        for (int b = 0; b < 4; b++) s1[b] = mlp_dot4(quad(H1 + (t.rt + 16 * b) * kPitch, r), x, s1[b]);
       }
+#pragma unroll
+      for (int b = 0; b < 4; b++) g1[b] += s1[b];
     }
     __syncthreads();
   }
-  for (int k = threadIdx.x; k < kParams; k += blockDim.x) atomicAdd(&grad[k], G[k]);
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    const int j = t.rt + 16 * b;
+#pragma unroll
+    for (int a = 0; a < 8; a++) atomicAdd(&grad[oW2 + (8 * t.ut + a) * kH + j], g2[a][b]);
+    atomicAdd(&grad[oW3 + t.ut * kH + j], g3[b]);
+    atomicAdd(&grad[t.ut < kIn ? oW1 + j * kIn + t.ut : oB1 + j], g1[b]);
+  }
+  if (tid < kH) atomicAdd(&grad[oB2 + tid], gb);
+  else if (tid < kH + kOut) atomicAdd(&grad[oB3 + tid - kH], gb);
 }
 
 __global__ void k_adam(int32_t np, float *__restrict__ p, float *__restrict__ g, float *__restrict__ m,
@@ -812,7 +971,7 @@ struct f3r_learned {
   int32_t loss_cap = 0;
   double *inv_ee = nullptr;       // 1 / ||e_p||^2 per pair
   int64_t steps = 0;
-  int grid_back = 0;              // persistent grid of the backward kernel
+  int grid_back = 0;              // persistent grid of the fp32 forward and backward kernels
   SysDev train;                   // the training system and its pairs
 };
 
@@ -832,7 +991,8 @@ Status forward(Context &c, const float *params, SysDev &s, int mode) {
     launch_k(c, k_mlp_infer_bf16, (int)std::min<int64_t>(cdiv(s.n, 64), (int64_t)c.sm_count * 8), 128, 0, c.stream,
              s.n, (const float *)s.feat, params, s.out);
   else
-    launch_k(c, k_mlp_forward, (int)cdiv(s.n, kRows), kRows, 0, c.stream, s.n, (const float *)s.feat, params, s.out);
+    launch_k(c, k_mlp_forward, (int)std::min<int64_t>(cdiv(s.n, kRows), (int64_t)c.sm_count * 2), kRows, kForwardSmem, c.stream, s.n,
+             (const float *)s.feat, params, s.out);
   const int g = (int)cdiv(s.n, 256);
   launch_k(c, k_correct, g, 256, 0, c.stream, s.n, (const int32_t *)s.zr, (const int32_t *)s.zs,
            (const double *)s.zv, (const float *)s.out, 0, s.zc);
@@ -891,6 +1051,7 @@ f3r_status f3r_learned_create(f3r_context *ctx, int32_t hidden, uint64_t seed, f
   for (float **b : {&L->p, &L->g, &L->m, &L->v}) F3R_TRY(c.alloc((void **)b, sizeof(float) * kParams));
   CUDA_TRY(cudaMemcpy(L->p, p.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice));
   for (float *b : {L->g, L->m, L->v}) CUDA_TRY(cudaMemset(b, 0, sizeof(float) * kParams));
+  CUDA_TRY(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForwardSmem));
   CUDA_TRY(cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBackSmem));
   CUDA_TRY(cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
   int per_sm = 0;
@@ -1059,8 +1220,8 @@ f3r_status f3r_learned_time_inference(f3r_learned *L, const f3r_csr *a, int32_t 
       launch_k(c, k_mlp_infer_bf16, (int)std::min<int64_t>(cdiv(s.n, 64), (int64_t)c.sm_count * 8), 128, 0,
                c.stream, s.n, (const float *)s.feat, (const float *)L->p, s.out);
     else
-      launch_k(c, k_mlp_forward, (int)cdiv(s.n, kRows), kRows, 0, c.stream, s.n, (const float *)s.feat,
-               (const float *)L->p, s.out);
+      launch_k(c, k_mlp_forward, (int)std::min<int64_t>(cdiv(s.n, kRows), (int64_t)c.sm_count * 2), kRows, kForwardSmem, c.stream,
+               s.n, (const float *)s.feat, (const float *)L->p, s.out);
     CUDA_TRY(cudaGetLastError());
     return F3R_SUCCESS;
   };
