@@ -2,7 +2,7 @@
 // dot products of w with up to 8 basis vectors, and the update, norm and Givens
 // step.
 //
-// They form exactly the sums of k_multidot_f32K and k_cgs_updateK (block.cuh,
+// They form exactly the sums of k_dotsK (blockdots.cuh) and k_cgs_updateK (block.cuh,
 // the K-column kernels whose columns must equal single solves): a logical grid
 // of up to 8 blocks of 256 threads an SM, each thread the 16-byte quads tid,
 // tid + stride, ... in order; warp butterflies; the 8 warps of a block in order;
@@ -203,33 +203,34 @@ __global__ void __launch_bounds__(256, 4)
 struct Givens8 {
   static constexpr int LD = kMaxDots1 + 1;
   float H[kMaxDots1 * LD], cs[kMaxDots1], sn[kMaxDots1], e[LD], y[kMaxDots1];
-  __device__ __forceinline__ void stage(const LevelK<float> &L, int j, int compute_y, const float *sh) {
-    const int t = threadIdx.x;
+  // column c's arrays by 64 threads t; sh[k * pitch]: the step's dots
+  __device__ __forceinline__ void stage(const LevelK<float> &L, int c, int j, int compute_y, const float *sh, int pitch,
+                                        int t) {
     if (t <= j) {
-      H[j * LD + t] = sh[t];
-      e[t] = L.e[t];
+      H[j * LD + t] = sh[t * pitch];
+      e[t] = L.e[c * L.vs + t];
       if (t < j) {
-        cs[t] = L.cs[t];
-        sn[t] = L.sn[t];
+        cs[t] = L.cs[c * L.vs + t];
+        sn[t] = L.sn[c * L.vs + t];
       }
     }
     if (compute_y && t < 64) {
       const int q = t / 8, i = t % 8;
-      if (q < j && i <= q) H[q * LD + i] = L.H[q * L.ldh + i];
+      if (q < j && i <= q) H[q * LD + i] = L.H[c * L.hs + q * L.ldh + i];
     }
   }
-  // thread 0, after a barrier
-  __device__ __forceinline__ void step(const LevelK<float> &L, int j, int compute_y, int *err, float nrm2) {
-    const GivensCtl<float> g{H, cs, sn, e, y, L.inv, nullptr, LD, j, compute_y, err};
+  // one thread, after a barrier
+  __device__ __forceinline__ void step(const LevelK<float> &L, int c, int j, int compute_y, int *err, float nrm2) {
+    const GivensCtl<float> g{H, cs, sn, e, y, L.inv + c, nullptr, LD, j, compute_y, err};
     givens_step<float>(g, nrm2);
-    float *Hc = L.H + (int64_t)j * L.ldh;
+    float *Hc = L.H + c * L.hs + (int64_t)j * L.ldh;
     for (int i = 0; i <= j + 1; i++) Hc[i] = H[j * LD + i];
-    L.cs[j] = cs[j];
-    L.sn[j] = sn[j];
-    L.e[j] = e[j];
-    L.e[j + 1] = e[j + 1];
+    L.cs[c * L.vs + j] = cs[j];
+    L.sn[c * L.vs + j] = sn[j];
+    L.e[c * L.vs + j] = e[j];
+    L.e[c * L.vs + j + 1] = e[j + 1];
     if (compute_y)
-      for (int i = 0; i <= j; i++) L.y[i] = y[i];
+      for (int i = 0; i <= j; i++) L.y[c * L.vs + i] = y[i];
   }
 };
 
@@ -312,10 +313,10 @@ __global__ void __launch_bounds__(256, 4)
     parts[blockIdx.x * L + threadIdx.x] = s;
   }
   if (!last_block1(gr.ticket)) return;
-  gs.stage(Lv, j, compute_y, sh);
+  if (threadIdx.x < 64) gs.stage(Lv, 0, j, compute_y, sh, 1, threadIdx.x);
   const float nrm2 = final_sums1<1>(parts, lgrid, 0, 1, 1, sw);
   if (threadIdx.x == 0) {
-    gs.step(Lv, j, compute_y, err, nrm2);
+    gs.step(Lv, 0, j, compute_y, err, nrm2);
     *gr.ticket = 0;
   }
 }

@@ -814,69 +814,6 @@ __global__ void __launch_bounds__(WARPS * 32, K == 1 ? 8 : 1) k_multidot_chunked
   if (threadIdx.x == 0) *gr.ticket = 0;
 }
 
-// H(j, k)(c) = <w(:, c), V(k)(:, c)> for nv <= MAXV basis vectors in fp32
-// (k_multidot_f32): rows in groups of 4 per thread, block-strided final stage
-template <int MAXV, int WARPS, int K>
-__global__ void __launch_bounds__(WARPS * 32) k_multidot_f32K(const float *__restrict__ w, Cols<float> V, int nv,
-                                                              int64_t n, GridRed gr, float *hcol, int64_t hstride) {
-  // basis vectors per pass: up to 32 values (single columns have k_dots1, blas1.cuh)
-  constexpr int CV = MAXV * K > 32 ? (32 / K > 0 ? 32 / K : 1) : MAXV;
-  constexpr int NQ = CV * K;
-  __shared__ float sred[WARPS][NQ];
-  float *part = static_cast<float *>(gr.partials);
-  const int ntot = nv * K;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x, tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nq4 = n / 4;
-  for (int k0 = 0; k0 < nv; k0 += CV) {
-    float a[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) a[q] = 0.0f;
-    // the 4 rows of a thread, RG at a time as one contiguous run of RG * K values
-    constexpr int RG = (4 * K <= 16) ? 4 : 1, E = RG * K;
-    for (int64_t q4 = tid; q4 < nq4; q4 += stride) {
-#pragma unroll
-      for (int g = 0; g < 4 / RG; g++) {
-        const int64_t i0 = 4 * q4 + g * RG;
-        float wv[E];
-        RowK<float, E>::load(w + i0 * K, wv);
-#pragma unroll
-        for (int v = 0; v < CV; v++) {
-          if (k0 + v < nv) {
-            float vv[E];
-            RowK<float, E>::load(V.p[k0 + v] + i0 * K, vv);
-#pragma unroll
-            for (int e = 0; e < E; e++) a[v * K + e % K] = __fmaf_rn(wv[e], vv[e], a[v * K + e % K]);
-          }
-        }
-      }
-    }
-    for (int64_t i = nq4 * 4 + tid; i < n; i += stride) {
-      float wv[K];
-      RowK<float, K>::load(w + i * K, wv);
-#pragma unroll
-      for (int v = 0; v < CV; v++) {
-        if (k0 + v < nv) {
-          float vv[K];
-          RowK<float, K>::load(V.p[k0 + v] + i * K, vv);
-#pragma unroll
-          for (int c = 0; c < K; c++) a[v * K + c] = __fmaf_rn(wv[c], vv[c], a[v * K + c]);
-        }
-      }
-    }
-    const int nq = min(CV, nv - k0) * K;
-    block_partials<float, NQ, WARPS>(a, nq, k0 * K, ntot, part, sred);
-  }
-  if (!last_block(gr.ticket)) return;
-  constexpr int QB = NQ < 16 ? NQ : 16;
-  for (int q0 = 0; q0 < ntot; q0 += QB) {
-    const int nq = min(QB, ntot - q0);
-    const float t = final_block_multi<float, WARPS, QB>(part, q0, nq, ntot);
-    const int q = q0 + (int)threadIdx.x;
-    if ((int)threadIdx.x < nq) hcol[(q % K) * hstride + q / K] = t;
-  }
-  if (threadIdx.x == 0) *gr.ticket = 0;
-}
-
 // shared memory of k_cgs_updateK's staging tiles: per warp 32 threads x N
 // rows x K values, each thread's run padded by 16 bytes (conflict-free
 // 16-byte reads)

@@ -24,7 +24,7 @@
 #include "internal.hpp"
 #include "kernels.cuh"
 #include "block.cuh"
-#include "blas1.cuh"
+#include "blockdots.cuh"
 #include "ilu.cuh"
 #include "objects.cuh"
 #include "trsv.hpp"
@@ -759,6 +759,7 @@ template <int K> struct Engine {
       // the Gram-Schmidt update's staging tiles (above 48 KB from K = 16)
       CUDA_TRY(cudaFuncSetAttribute(k_cgs_updateK<float, 8, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)cgs_stage_bytes<float, 8, K>()));
+      CUDA_TRY(cudaFuncSetAttribute(k_dotsK<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dots_stage_bytes<K>()));
       CUDA_TRY(cudaFuncSetAttribute(k_cgs_updateK<double, 8, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)cgs_stage_bytes<double, 8, K>()));
       if (S.mm) {
@@ -1025,12 +1026,8 @@ template <int K> struct Engine {
         return;
       }
     } else {
-      if (nv <= 4) {
-        launch_k(C(), k_multidot_f32K<4, 8, K>, g4, 256, 0, C().stream, wv, Vc, nv, (int64_t)n, w.gr, hcol, hs);
-        return;
-      }
-      if (nv <= 8) {
-        launch_k(C(), k_multidot_f32K<8, 8, K>, g4, 256, 0, C().stream, wv, Vc, nv, (int64_t)n, w.gr, hcol, hs);
+      if (nv <= kMaxDots1) {
+        launch_k(C(), k_dotsK<K>, g4, 256, dots_stage_bytes<K>(), C().stream, wv, Vc, nv, (int64_t)n, w.gr, hcol, hs);
         return;
       }
     }
