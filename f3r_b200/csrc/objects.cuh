@@ -190,11 +190,7 @@ inline bool launch_pattern(Context &c, const V *val, const DevPattern &d, const 
   if (p.stages == 0) return false;
   PatArgs a = d.a;
   a.stages = p.stages;
-  // the first tile whose windows pass x's last whole 16-byte unit
-  int32_t hi = 0;
-  for (int w = 0; w < a.nwin; w++) hi = std::max(hi, a.win[w].lo + a.win[w].len);
-  const int64_t per = 16 / (int64_t)sizeof(X), nfl = a.n / per * per;
-  a.tail_tile = nfl == a.n ? a.ntiles : (int32_t)std::max<int64_t>(0, (nfl - hi) / a.tile);
+  a.tail_tile = pattern_tail(a, 16 / (int64_t)sizeof(X));
   const int64_t work = std::max<int64_t>(a.ntiles, cdiv(a.ngroups, d.warps));
   launch_k(c, k_sell_pattern<V, X, Epi>, (unsigned)std::min<int64_t>(work, (int64_t)c.sm_count * p.ctas), (d.warps + 1) * 32,
            p.smem, c.stream, a, d.tab(val), d.vals(val), x, epi, epi_vec4(epi) ? 1 : 0, c.err);

@@ -65,8 +65,9 @@ struct Pattern {
 struct Layout {
   PatArgs a{};
   int warps = 0;
+  PatArgs ab{};  // tiles of one block
   std::vector<Pattern> pats;
-  std::vector<int32_t> soff;  // of every run, pattern by pattern
+  std::vector<int32_t> soff, soffb;  // of every run, pattern by pattern
   std::vector<uint8_t> blk, live;
   std::vector<int32_t> irow, iptr, icol;
   std::vector<double> ival;
@@ -90,6 +91,45 @@ bool make_runs(Pattern &p) {
     k += len;
   }
   return w > 0 && (int)p.runs.size() <= kPatRuns;
+}
+
+// The windows of x that tiles of a.tile rows read, and every run's place in the
+// stage; offsets less than a tile apart share a window (the rows between cost
+// less than a window of their own).
+bool windows(const std::vector<Pattern> &pats, PatArgs &a, std::vector<int32_t> &soff) {
+  std::vector<int32_t> offs;
+  for (const Pattern &q : pats)
+    for (const Run &r : q.runs) {
+      offs.push_back(r.d);
+      offs.push_back(r.d + r.len - 1);
+    }
+  std::sort(offs.begin(), offs.end());
+  auto down = [](int64_t v) { return (int32_t)((v >= 0 ? v : v - (kPatUnit - 1)) / kPatUnit * kPatUnit); };
+  std::vector<std::pair<int32_t, int32_t>> win;
+  for (const int32_t e : offs) {
+    if (!win.empty() && (int64_t)e - win.back().second < a.tile) win.back().second = e;
+    else win.emplace_back(e, e);
+  }
+  if ((int)win.size() > kPatWindows) return false;
+  a.nwin = (int32_t)win.size();
+  int64_t elems = 0;
+  for (int w = 0; w < a.nwin; w++) {
+    const int32_t lo = down(win[w].first);
+    // up to 8 elements past the last row's last one are read (and not used)
+    const int64_t len = cdiv((int64_t)a.tile + win[w].second - lo + 9, kPatUnit) * kPatUnit;
+    if (elems + len >= kPatLong) return false;
+    a.win[w] = PatWindow{lo, (int32_t)len, (int32_t)elems};
+    elems += len;
+  }
+  a.elems = (int32_t)elems;
+  for (const Pattern &q : pats)
+    for (const Run &r : q.runs)
+      for (int w = 0; w < a.nwin; w++)
+        if (r.d >= win[w].first && r.d <= win[w].second) {
+          soff.push_back(a.win[w].base + r.d - a.win[w].lo);
+          break;
+        }
+  return true;
 }
 
 template <typename T> Status put(Context &c, DevPattern &p, T **d, const T *h, size_t count) {
@@ -118,27 +158,32 @@ template <typename T> Status rounded(Context &c, const std::vector<double> &v, s
 
 // the pattern table and the other rows' values in type V
 template <typename V>
-Status put_values(Context &c, DevPattern &p, const std::vector<Pattern> &pats, const std::vector<int32_t> &soff,
-                  const std::vector<double> &ival, PatRun<V> **tab, V **val) {
+Status put_values(Context &c, DevPattern &p, const Layout &o, PatRun<V> *(&tab)[2], V **val) {
+  const std::vector<Pattern> &pats = o.pats;
+  const std::vector<double> &ival = o.ival;
   std::vector<double> flat;
   for (const Pattern &q : pats)
     for (const Run &r : q.runs) flat.insert(flat.end(), r.v, r.v + 3);
   std::vector<V> rv;
   F3R_TRY(rounded<V>(c, flat, rv));
-  std::vector<PatRun<V>> t((size_t)p.a.np * p.a.stride);
-  std::memset((void *)t.data(), 0, t.size() * sizeof(PatRun<V>));
-  size_t at = 0;
-  for (size_t q = 0; q < pats.size(); q++) {
-    PatRun<V> *o = t.data() + q * p.a.stride;
-    bool lng = true;
-    for (const Run &r : pats[q].runs) lng = lng && r.len == 3;
-    o[0].at = (int32_t)pats[q].runs.size() | (pats[q].pad ? kPatPadded : 0) | (lng ? kPatAllLong : 0);
-    for (size_t k = 0; k < pats[q].runs.size(); k++, at++) {
-      o[k + 1].at = soff[at] | (pats[q].runs[k].len == 3 ? kPatLong : 0);
-      for (int j = 0; j < 3; j++) o[k + 1].v[j] = rv[3 * at + j];
+  for (int i = 0; i < 2; i++) {
+    const std::vector<int32_t> &soff = i ? o.soffb : o.soff;
+    std::vector<PatRun<V>> t((size_t)p.a.np * p.a.stride);
+    std::memset((void *)t.data(), 0, t.size() * sizeof(PatRun<V>));
+    size_t at = 0;
+    for (size_t q = 0; q < pats.size(); q++) {
+      PatRun<V> *r = t.data() + q * p.a.stride;
+      bool lng = true;
+      for (const Run &e : pats[q].runs) lng = lng && e.len == 3;
+      r[0].at = (int32_t)pats[q].runs.size() | (pats[q].pad ? kPatPadded : 0) | (lng ? kPatAllLong : 0);
+      for (size_t k = 0; k < pats[q].runs.size(); k++, at++) {
+        r[k + 1].at = soff[at] | (pats[q].runs[k].len == 3 ? kPatLong : 0);
+        for (int j = 0; j < 3; j++) r[k + 1].v[j] = rv[3 * at + j];
+      }
     }
+    F3R_TRY(put(c, p, &tab[i], t.data(), t.size()));
+    CUDA_TRY(cudaStreamSynchronize(c.stream));  // t is read until then
   }
-  F3R_TRY(put(c, p, tab, t.data(), t.size()));
   F3R_TRY(c.alloc((void **)val, std::max<size_t>(ival.size(), 1) * sizeof(V)));
   p.allocs.push_back((void *)*val);
   if (!ival.empty()) {
@@ -249,44 +294,12 @@ static bool layout(const SellHost &h, int sm_count, Layout &o) {
   a.ntiles = (int32_t)cdiv(n, a.tile);
   a.np = (int32_t)pats.size();
   a.stride = 1;
-  std::vector<int32_t> offs;
-  for (const Pattern &q : pats) {
-    a.stride = std::max<int32_t>(a.stride, (int32_t)q.runs.size() + 1);
-    for (const Run &r : q.runs) {
-      offs.push_back(r.d);
-      offs.push_back(r.d + r.len - 1);
-    }
-  }
-  std::sort(offs.begin(), offs.end());
-  // offsets less than a tile apart share a window: the rows between cost less than a window of their own
-  auto down = [](int32_t v) { return (int32_t)(v >= 0 ? v / kPatUnit * kPatUnit : -((-(int64_t)v + kPatUnit - 1) / kPatUnit * kPatUnit)); };
-  std::vector<std::pair<int32_t, int32_t>> win;
-  for (const int32_t e : offs) {
-    if (!win.empty() && (int64_t)e - win.back().second < a.tile) win.back().second = e;
-    else win.emplace_back(e, e);
-  }
-  if ((int)win.size() > kPatWindows) return false;
-  a.nwin = (int32_t)win.size();
-  int64_t elems = 0;
-  for (int w = 0; w < a.nwin; w++) {
-    const int32_t lo = down(win[w].first);
-    // up to 8 elements past the last row's last one are read (and not used)
-    const int64_t len = cdiv((int64_t)a.tile + win[w].second - lo + 9, kPatUnit) * kPatUnit;
-    if (len > 1 << 20) return false;
-    a.win[w] = PatWindow{lo, (int32_t)len, (int32_t)elems};
-    elems += len;
-  }
-  a.elems = (int32_t)elems;
-  if (elems >= kPatLong) return false;
+  for (const Pattern &q : pats) a.stride = std::max<int32_t>(a.stride, (int32_t)q.runs.size() + 1);
+  o.ab = a;
+  o.ab.tile = kPatBlock;
+  o.ab.ntiles = nblk;
+  if (!windows(pats, a, o.soff) || !windows(pats, o.ab, o.soffb)) return false;
   if (pattern_shape(a, o.warps, 2, sizeof(PatRun<__half>)).stages == 0) return false;
-  std::vector<int32_t> &soff = o.soff;
-  for (const Pattern &q : pats)
-    for (const Run &r : q.runs)
-      for (int w = 0; w < a.nwin; w++)
-        if (r.d >= win[w].first && r.d <= win[w].second) {
-          soff.push_back(a.win[w].base + r.d - a.win[w].lo);
-          break;
-        }
   // the other rows, grouped by width
   std::vector<int32_t> rest;
   for (int64_t r = 0; r < n; r++)
@@ -345,9 +358,16 @@ Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d
   p.a.irow = rd;
   p.a.iptr = pd;
   p.a.icol = cd;
-  if (dtype_mask & (1 << F3R_F64)) F3R_TRY(put_values<double>(c, p, o.pats, o.soff, o.ival, &p.t64, &p.v64));
-  if (dtype_mask & (1 << F3R_F32)) F3R_TRY(put_values<float>(c, p, o.pats, o.soff, o.ival, &p.t32, &p.v32));
-  if (dtype_mask & (1 << F3R_F16)) F3R_TRY(put_values<__half>(c, p, o.pats, o.soff, o.ival, &p.t16, &p.v16));
+  p.ab = o.ab;
+  p.ab.ngroups = p.a.ngroups;
+  p.ab.blk = bd;
+  p.ab.live = ld;
+  p.ab.irow = rd;
+  p.ab.iptr = pd;
+  p.ab.icol = cd;
+  if (dtype_mask & (1 << F3R_F64)) F3R_TRY(put_values<double>(c, p, o, p.t64, &p.v64));
+  if (dtype_mask & (1 << F3R_F32)) F3R_TRY(put_values<float>(c, p, o, p.t32, &p.v32));
+  if (dtype_mask & (1 << F3R_F16)) F3R_TRY(put_values<__half>(c, p, o, p.t16, &p.v16));
   CUDA_TRY(cudaStreamSynchronize(c.stream));
   d.pat = dp.release();
   return F3R_SUCCESS;

@@ -355,16 +355,18 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
 struct DevPattern {
   PatArgs a{};
   int warps = 0;
-  PatRun<double> *t64 = nullptr;
-  PatRun<float> *t32 = nullptr;
-  PatRun<__half> *t16 = nullptr;
+  PatArgs ab{};  // for tiles of one block (patblock.cuh)
+  // the patterns' records, for a's tiles and for ab's
+  PatRun<double> *t64[2] = {nullptr, nullptr};
+  PatRun<float> *t32[2] = {nullptr, nullptr};
+  PatRun<__half> *t16[2] = {nullptr, nullptr};
   double *v64 = nullptr;
   float *v32 = nullptr;
   __half *v16 = nullptr;
   std::vector<void *> allocs;
-  const PatRun<double> *tab(const double *) const { return t64; }
-  const PatRun<float> *tab(const float *) const { return t32; }
-  const PatRun<__half> *tab(const __half *) const { return t16; }
+  const PatRun<double> *tab(const double *, int i = 0) const { return t64[i]; }
+  const PatRun<float> *tab(const float *, int i = 0) const { return t32[i]; }
+  const PatRun<__half> *tab(const __half *, int i = 0) const { return t16[i]; }
   const double *vals(const double *) const { return v64; }
   const float *vals(const float *) const { return v32; }
   const __half *vals(const __half *) const { return v16; }
@@ -385,6 +387,13 @@ struct PatShape {
 // and 6.1; fp32 8.4 and 6.6, fp64 12.4 and 7.9; at 48^3 no gain is left).
 inline int64_t pattern_rows(int sm_count, int height, size_t sv) {
   return (int64_t)sm_count * (height == 64 && sv == 2 ? 2048 : 1024);
+}
+// the first tile whose windows pass the last of n rows that whole units of `per` rows bring
+inline int32_t pattern_tail(const PatArgs &a, int64_t per) {
+  int64_t hi = 0;
+  for (int w = 0; w < a.nwin; w++) hi = std::max<int64_t>(hi, (int64_t)a.win[w].lo + a.win[w].len);
+  const int64_t nfl = a.n / per * per;
+  return nfl == a.n ? a.ntiles : (int32_t)std::max<int64_t>(0, (nfl - hi) / a.tile);
 }
 inline PatShape pattern_shape(const PatArgs &a, int warps, size_t sx, size_t st) {
   const size_t one = (size_t)a.elems * sx, table = (size_t)a.np * a.stride * st, sm = 227 * 1024;
