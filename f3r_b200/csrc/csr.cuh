@@ -2,33 +2,32 @@
 // option of the solver and F3R_SELL_CSR matrices).  The reference's CSR
 // operate is matrix/csr.hpp's; its GPU drivers use SELL<32>.
 //
-// The launch geometry is the packed SELL kernel's: WARPS warps per CTA, one
-// CTA per SM at most, warp w of CTA b takes the 32-row groups b*WARPS + w,
-// + gridDim*WARPS, ...; lane l owns row 32 g + l.  Each warp streams the
-// contiguous CSR range of its groups through a two-stage shared-memory ring
-// in tiles of up to kCsrTile entries: the tile's byte range, widened to
-// 16-byte boundaries, is copied with 16-byte cp.async (the next tile is in
-// flight while the current one is summed), and each lane sums its own row
-// sequentially in column order, kCsrBatch gathers at a time.  So every row's
-// sum, every thread's partial dot products and every CTA's partials are the
-// packed sigma = 1 SELL kernel's, bit for bit (SELL's padding adds exact
-// zeros).  The value and index arrays carry kCsrPad elements of padding, so
-// the widened copies stay inside their allocations.
+// A warp takes a group of 32 rows, lane l row 32 g + l.  The group's contiguous
+// CSR range (in tiles of T entries) is widened to 16-byte boundaries and copied
+// to shared memory with 16-byte cp.async, and each lane sums its own row in
+// column order, B gathers at a time: the packed SELL layout's sums bit for bit
+// (SELL's padding adds exact zeros).  The value and index arrays carry kCsrPad
+// elements of padding, so the widened copies stay inside their allocations.
+//
+// What bounds it is each group's chain of waits (row pointers, copy, one or two
+// rounds of gathers), so the more groups an SM holds the better: blocks of 4
+// warps that the hardware schedules as others finish, one tile of shared memory a
+// warp, and tiles of kCsrShort entries where every group fits them (rows of at
+// most 8 entries: 64 warps an SM; 128^3 7-point, fp32: 27.5 us, 52.4 with
+// kCsrWide), of kCsrWide otherwise.  Against 24 persistent warps an SM with a
+// two-stage ring of 512 entries: 27-point, fp16, 40^3 7.4 -> 4.1 us, 64^3 17.5 ->
+// 9.4, 128^3 109 -> 74; 7-point 64^3 6.5 -> 4.4, 200^3 147 -> 100.
 #pragma once
 
 #include "sell.cuh"
 
 namespace f3r {
 
-constexpr int kCsrTile = 512;  // entries per tile
-constexpr int kCsrBatch = 8;   // gathers in flight per lane
-constexpr int kCsrPad = 16;    // elements of padding after the value and index arrays
+constexpr int kCsrWide = 1024, kCsrShort = 256;  // entries a tile
+constexpr int kCsrWarps = 4;                     // warps a block
+constexpr int kCsrPad = 16;                      // elements of padding after the value and index arrays
 
-template <typename V> constexpr uint32_t csr_vstage() { return kCsrTile * sizeof(V) + 32; }
-constexpr uint32_t csr_istage() { return kCsrTile * 4 + 32; }
-template <typename V> constexpr size_t csr_smem_bytes() {
-  return (size_t)SellCfg<V, int32_t>::WARPS * 2 * (csr_vstage<V>() + csr_istage());
-}
+template <typename V, int T> constexpr uint32_t csr_tile_bytes() { return T * sizeof(V) + 32 + T * 4 + 32; }
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -38,96 +37,50 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <typename V, typename X, typename Epi, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 1)
-    k_csr_cfg(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi, int *) {
+template <typename V, typename X, typename Epi, int T>
+__global__ void __launch_bounds__(kCsrWarps * 32)
+    k_csr_group(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
-  constexpr uint32_t VS = csr_vstage<V>(), IS = csr_istage();
+  constexpr int B = T == kCsrShort ? 8 : 16;  // gathers in flight per lane
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char *vbuf = smem + (size_t)warp * 2 * (VS + IS);  // stage s: values at s * VS
-  unsigned char *ibuf = vbuf + 2 * VS;                       // stage s: indices at s * IS
-  typename Epi::Red dots[Epi::NV > 0 ? Epi::NV : 1];
-#pragma unroll
-  for (int k = 0; k < (Epi::NV > 0 ? Epi::NV : 1); k++) dots[k] = 0;
-  const int TW = gridDim.x * WARPS;
-  auto gend = [&](int c) { return A.rptr[min((int64_t)c * 32 + 32, (int64_t)A.n)]; };
-  // first tile of the first non-empty group at or after c (stepping TW)
-  auto first_from = [&](int c, int &pc, int32_t &pt) {
-    for (; c < A.nslices; c += TW) {
-      const int32_t b = A.rptr[(int64_t)c * 32];
-      if (b < gend(c)) {
-        pc = c;
-        pt = b;
-        return true;
-      }
-    }
-    return false;
-  };
-  // copies tile (c, t0) into stage s; returns the element offsets of its first entry
-  auto issue = [&](int s, int c, int32_t t0, int &voff, int &ioff) {
-    const int32_t cnt = min(kCsrTile, gend(c) - t0);
-    const char *vs = reinterpret_cast<const char *>(val);
-    const size_t b0 = (size_t)t0 * sizeof(V), a0 = b0 & ~(size_t)15;
-    const size_t a1 = ((size_t)(t0 + cnt) * sizeof(V) + 15) & ~(size_t)15;
-    for (size_t k = lane; k < (a1 - a0) / 16; k += 32) cp_async16(vbuf + s * VS + k * 16, vs + a0 + k * 16);
-    const char *is = reinterpret_cast<const char *>(A.col);
-    const size_t c0 = (size_t)t0 * 4, d0 = c0 & ~(size_t)15, d1 = ((size_t)(t0 + cnt) * 4 + 15) & ~(size_t)15;
-    for (size_t k = lane; k < (d1 - d0) / 16; k += 32) cp_async16(ibuf + s * IS + k * 16, is + d0 + k * 16);
+  const int64_t g = (int64_t)blockIdx.x * kCsrWarps + warp, r = g * 32 + lane;
+  if (g >= A.nslices) return;
+  unsigned char *vbuf = smem + (size_t)warp * csr_tile_bytes<V, T>(), *ibuf = vbuf + T * sizeof(V) + 32;
+  const bool live = r < A.n;
+  const int32_t rb = A.rptr[live ? r : A.n], re = A.rptr[live ? r + 1 : A.n];
+  const int32_t gb = __shfl_sync(0xffffffffu, rb, 0), ge = __shfl_sync(0xffffffffu, re, 31);
+  typename Epi::Pre pre{};
+  if (live) pre = epi.load(r);
+  Acc acc = 0;
+  for (int32_t t0 = gb; t0 < ge; t0 += T) {
+    const int cnt = min(T, ge - t0);
+    // the tile's byte ranges widened to 16-byte units (the arrays carry kCsrPad elements)
+    const size_t b0 = (size_t)t0 * sizeof(V), a0 = b0 & ~(size_t)15, c0 = (size_t)t0 * 4, d0 = c0 & ~(size_t)15;
+    const int nv = (int)((b0 + cnt * sizeof(V) + 15 - a0) / 16), ni = (int)((c0 + (size_t)cnt * 4 + 15 - d0) / 16);
+    const char *vs = reinterpret_cast<const char *>(val) + a0, *is = reinterpret_cast<const char *>(A.col) + d0;
+    for (int k = lane; k < ni; k += 32) cp_async16(ibuf + k * 16, is + k * 16);
+    for (int k = lane; k < nv; k += 32) cp_async16(vbuf + k * 16, vs + k * 16);
     cp_async_commit();
-    voff = (int)((b0 - a0) / sizeof(V));
-    ioff = (int)((c0 - d0) / 4);
-  };
-  int pc = 0, stage = 0, vo0 = 0, vo1 = 0, io0 = 0, io1 = 0;  // per stage: offsets of the first entry
-  int32_t pt = 0;
-  // the prefetch cursor (pc, pt): the last tile issued
-  if (first_from(blockIdx.x * WARPS + warp, pc, pt)) issue(0, pc, pt, vo0, io0);
-  for (int cs = blockIdx.x * WARPS + warp; cs < A.nslices; cs += TW) {
-    const int64_t r = (int64_t)cs * 32 + lane;
-    const bool live = r < A.n;
-    const int32_t rb = live ? A.rptr[r] : 0, re = live ? A.rptr[r + 1] : 0;
-    const int32_t gb = A.rptr[(int64_t)cs * 32], ge = gend(cs);
-    typename Epi::Pre pre{};
-    if (live) pre = epi.load(r);
-    Acc acc = 0;
-    for (int32_t t0 = gb; t0 < ge; t0 += kCsrTile) {
-      // this tile sits in `stage`; put the next one in flight in the other stage
-      bool next;
-      if (pt + kCsrTile < gend(pc)) {
-        pt += kCsrTile;
-        next = true;
-      } else {
-        next = first_from(pc + TW, pc, pt);
-      }
-      if (next) {
-        if (stage) issue(0, pc, pt, vo0, io0);
-        else issue(1, pc, pt, vo1, io1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
-      __syncwarp();
-      const V *sv = reinterpret_cast<const V *>(vbuf + stage * VS) + (stage ? vo1 : vo0);
-      const int32_t *sc = reinterpret_cast<const int32_t *>(ibuf + stage * IS) + (stage ? io1 : io0);
-      const int cnt = min(kCsrTile, ge - t0);
-      const int lo = max(rb, t0) - t0, hi = min(re, t0 + cnt) - t0;
-      // the row's terms in column order; the last batch is masked, not reordered
-      for (int k = lo; k < hi; k += kCsrBatch) {
-        Acc xv[kCsrBatch];
+    cp_async_wait<0>();
+    __syncwarp();
+    const V *sv = reinterpret_cast<const V *>(vbuf + (b0 - a0));
+    const int32_t *sc = reinterpret_cast<const int32_t *>(ibuf + (c0 - d0));
+    const int lo = max(rb, t0) - t0, hi = min(re, t0 + cnt) - t0;
+    for (int k = lo; k < hi; k += B) {
+      Acc xv[B];
 #pragma unroll
-        for (int e = 0; e < kCsrBatch; e++)
-          if (k + e < hi) xv[e] = to_acc<Acc>(__ldg(x + sc[k + e]));
+      for (int e = 0; e < B; e++)
+        if (k + e < hi) xv[e] = to_acc<Acc>(__ldg(x + sc[k + e]));
 #pragma unroll
-        for (int e = 0; e < kCsrBatch; e++)
-          if (k + e < hi) acc = fmaT(to_acc<Acc>(sv[k + e]), xv[e], acc);
-      }
-      __syncwarp();  // every lane is done with this stage before it is refilled
-      stage ^= 1;
+      for (int e = 0; e < B; e++)
+        if (k + e < hi) acc = fmaT(to_acc<Acc>(sv[k + e]), xv[e], acc);
     }
-    if (live) epi.row(r, acc, pre, dots);
+    __syncwarp();  // every lane is done with the tile before it is refilled
   }
-  epi.template finish<WARPS>(dots);
+  typename Epi::Red none[1];
+  if (live) epi.row(r, acc, pre, none);
 }
 
 }  // namespace f3r

@@ -141,8 +141,8 @@ inline Status sell_attr(Context &c) {
     F3R_TRY((sell_attr_one<V, X, Epi, uint16_t>()));
     F3R_TRY((sell_attr_one<V, X, Epi, AlignedIdx>()));
     F3R_TRY((sell_attr_one<V, X, Epi, AllAlignedIdx>()));
-    CUDA_TRY(cudaFuncSetAttribute(k_csr_cfg<V, X, Epi, SellCfg<V, int32_t>::WARPS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csr_smem_bytes<V>()));
+    CUDA_TRY(cudaFuncSetAttribute(k_csr_group<V, X, Epi, kCsrWide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kCsrWarps * csr_tile_bytes<V, kCsrWide>())));
     using C64 = Sell64Cfg<V>;
     CUDA_TRY(cudaFuncSetAttribute(k_sell64<V, X, Epi, C64::WARPS, C64::STAGES, C64::KC>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sell64_smem_bytes<V>()));
@@ -228,10 +228,13 @@ inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x
     launch_k(c, k_sell64<V, X, Epi, C64::WARPS, C64::STAGES, C64::KC>, grid, C64::WARPS * 32, sell64_smem_bytes<V>(),
              c.stream, val, A, x, epi, c.err);
   } else if (A.rptr) {
-    // the packed kernel's geometry (rows per thread, CTAs), so sums and partials match it
-    constexpr int W = SellCfg<V, int32_t>::WARPS;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(A.nslices, W), c.sm_count));
-    launch_k(c, k_csr_cfg<V, X, Epi, W>, grid, W * 32, csr_smem_bytes<V>(), c.stream, val, A, x, epi, c.err);
+    const unsigned grid = (unsigned)cdiv(A.nslices, kCsrWarps);
+    if (A.max_width * 32 <= kCsrShort)
+      launch_k(c, k_csr_group<V, X, Epi, kCsrShort>, grid, kCsrWarps * 32, kCsrWarps * csr_tile_bytes<V, kCsrShort>(),
+               c.stream, val, A, x, epi);
+    else
+      launch_k(c, k_csr_group<V, X, Epi, kCsrWide>, grid, kCsrWarps * 32, kCsrWarps * csr_tile_bytes<V, kCsrWide>(),
+               c.stream, val, A, x, epi);
   } else if (A.xoff) launch_sell_one<V, X, Epi, AlignedIdx>(c, val, A, x, epi);
   else if (A.cbase && !A.dcol) launch_sell_one<V, X, Epi, AllAlignedIdx>(c, val, A, x, epi);
   else if (A.dcol) launch_sell_one<V, X, Epi, uint16_t>(c, val, A, x, epi);

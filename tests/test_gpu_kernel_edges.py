@@ -81,6 +81,27 @@ def test_products_bitexact_across_the_rules(ctx, kind, grid, kw):
     S.close()
 
 
+@pytest.mark.parametrize("n,lo,hi", [(1, 1, 1), (97, 0, 8), (64, 8, 8), (131, 9, 9), (70, 30, 70), (33, 0, 33)])
+def test_csr_tiles_bitexact(ctx, n, lo, hi):
+    """groups of 32 rows that fit the short tile, fill it, fit the wide one or
+    need several, empty rows and a ragged last group among them"""
+    rng = np.random.default_rng(n)
+    cnt = np.minimum(rng.integers(lo, hi + 1, n), n)
+    r = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    i = np.concatenate([np.sort(rng.choice(n, c, replace=False)) for c in cnt] or [[]]).astype(np.int32)
+    v = rng.standard_normal(len(i))
+    S = F.Sell(ctx, F.HostMatrix.from_csr(r, i, v, n), csr=True)
+    x = rng.standard_normal(n)
+    for vt, dt, tdt, ov in ((F.F64, np.float64, torch.float64, O.DT_F64), (F.F32, np.float32, torch.float32, O.DT_F32),
+                            (F.F16, np.float16, torch.float16, O.DT_F16)):
+        y = torch.zeros(n, dtype=tdt, device="cuda")
+        S.operate(torch.from_numpy(x.astype(dt)).cuda(), y, val_t=vt)
+        torch.cuda.synchronize()
+        want = O.spmv(r, i, v, x.astype(dt), ov, ov, O.DT_F64 if vt == F.F64 else O.DT_F32)
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
+    S.close()
+
+
 @pytest.mark.parametrize("grid", [(13, 11, 7), (32, 32, 32), (70, 69, 63), (97, 90, 71)])
 @pytest.mark.parametrize("m2,m3", [(8, 4), (3, 8), (5, 0)])
 def test_single_column_levels_are_the_block_kernels(ctx, grid, m2, m3):
