@@ -117,6 +117,7 @@ __device__ __forceinline__ float final_sums1(const float *part, int lgrid, int q
 template <int NV, int L>
 __global__ void __launch_bounds__(256, 4)
     k_dots1(const float *__restrict__ w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, float *__restrict__ hcol) {
+  stream_order();
   __shared__ float sred[8][L * NV];
   __shared__ float sw[8][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -240,6 +241,7 @@ template <int NV, int L>
 __global__ void __launch_bounds__(256, 4)
     k_cgs1(float *__restrict__ w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, LevelK<float> Lv, int j,
            int compute_y, int *err) {
+  stream_order();
   __shared__ float sh[kMaxDots1], ssc[kMaxDots1];
   __shared__ float sred[8][L];
   __shared__ float sw[8][1];
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(256, 4)
 // nz <= 8 columns, widened exactly, MULMV order
 __global__ void __launch_bounds__(256) k_zy1(const __half *__restrict__ Z, int64_t ldz, const float *__restrict__ y, int nz,
                                              float *__restrict__ out, int64_t n) {
+  stream_order();
   __shared__ float sy[kMaxDots1];
   if ((int)threadIdx.x < nz) sy[threadIdx.x] = y[threadIdx.x];
   __syncthreads();

@@ -997,6 +997,7 @@ template <int WARPS, int K>
 __global__ void __launch_bounds__(WARPS * 32) k_rich_weightK(const __half *__restrict__ tmp,
                                                              const __half *__restrict__ other, int64_t n,
                                                              GridRed gr, RichState *rs, int k) {
+  stream_order();
   __shared__ float sred[WARPS][2 * K];
   float d[2 * K];
 #pragma unroll
@@ -1060,6 +1061,7 @@ template <int R, typename F> __device__ __forceinline__ void for_row_groups(int6
 template <int K>
 __global__ void k_level2_enterK(double *const *__restrict__ in_slot, const double *__restrict__ inv,
                                 float *__restrict__ v0, float *e, int64_t e_stride, int64_t n) {
+  stream_order();
   double *in = *in_slot;
   double s[K];
 #pragma unroll
@@ -1085,6 +1087,7 @@ __global__ void k_level2_enterK(double *const *__restrict__ in_slot, const doubl
 template <typename T, typename Out, bool ACCUM, int K, typename ZT = T>
 __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_zyK(Cols<ZT> Z, const T *__restrict__ y, int64_t y_stride, int nz, Out *out_direct,
                       Out *const *out_slot, uint32_t mask, int64_t n) {
+  stream_order();
   __shared__ T sy[K][kMaxCols];
   for (int t = threadIdx.x; t < nz * K; t += blockDim.x) {
     const int c = t / nz, k = t % nz;
@@ -1152,6 +1155,7 @@ template <bool SCALE_BY_OME, int K, bool MM = false>
 __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK(float *__restrict__ in, const float *__restrict__ in_inv, float sc, DiagPre M,
                                    __half *__restrict__ hin, __half *__restrict__ hout,
                                    const RichState *__restrict__ rs, float *e_set, int64_t e_stride, int64_t n, bool store) {
+  stream_order();
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   float om[K], s[K];
 #pragma unroll
@@ -1173,6 +1177,7 @@ __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK
 template <int K>
 __global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict__ in_inv, float sc,
                                 __half *__restrict__ hin, float *e_set, int64_t e_stride, int64_t n, bool store) {
+  stream_order();
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   for_row_groups<RowsPer<K>::R>(n, [&](int64_t i0, auto rows) {
     constexpr int E = decltype(rows)::value * K;
@@ -1192,6 +1197,7 @@ __global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict_
 // hout(:, c) = fp16(hout * fp16(om_c[0])) (k_rich_scale_om)
 template <int K>
 __global__ void k_rich_scale_omK(__half *__restrict__ hout, const RichState *__restrict__ rs, int64_t n) {
+  stream_order();
   float om[K];
 #pragma unroll
   for (int c = 0; c < K; c++) om[c] = h2f(f2h(rs[c].om[0]));
@@ -1211,6 +1217,7 @@ template <int K>
 __global__ void k_rich_axpyK(__half *__restrict__ hout, const __half *__restrict__ t2,
                              const RichState *__restrict__ rs, int k, int use_ome, float *__restrict__ out, float isc,
                              int64_t n, __half *__restrict__ out16) {
+  stream_order();
   float om[K];
 #pragma unroll
   for (int c = 0; c < K; c++) om[c] = use_ome ? h2f(rs[c].ome[k]) : rs[c].om[k];
@@ -1234,6 +1241,7 @@ __global__ void k_rich_axpyK(__half *__restrict__ hout, const __half *__restrict
 // out = fp32(hout) / sc (k_rich_exit)
 template <int K>
 __global__ void k_rich_exitK(const __half *__restrict__ hout, float *__restrict__ out, float isc, int64_t n) {
+  stream_order();
   for_row_groups<RowsPer<K>::R>(n, [&](int64_t i0, auto rows) {
     constexpr int E = decltype(rows)::value * K;
     float h[E];

@@ -40,6 +40,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 template <typename V, typename X, typename Epi, int T>
 __global__ void __launch_bounds__(kCsrWarps * 32)
     k_csr_group(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+  stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
   constexpr int B = T == kCsrShort ? 8 : 16;  // gathers in flight per lane

@@ -78,6 +78,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
   }
   return true;
 }
+// Start of a kernel that may be launched while its predecessor still runs
+// (Context::overlap): waits until the predecessor has finished and its writes are
+// visible, then lets the successor be launched.  Nothing before it may touch
+// memory that another kernel of the stream writes or reads.  No effect in an
+// ordinary launch.
+__device__ __forceinline__ void stream_order() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 // L2 policy for streamed-once data (matrix values and indices): evict first,
 // so the gathered vector stays resident in L2.
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {

@@ -113,6 +113,7 @@ __device__ __forceinline__ void direct_aligned_rows(const V *val, const DevSell 
 template <typename V, typename X, typename Epi, int H, int R>
 __global__ void __launch_bounds__(kDirectThreads)
     k_sell_direct_aligned(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+  stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, r0 = t / 32 * (32 * R) + t % 32;
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(kDirectThreads)
 template <typename V, typename X, typename Epi, int H>
 __global__ void __launch_bounds__(kDirectThreads)
     k_sell_direct_mixed(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+  stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(kDirectThreads)
 template <typename V, typename X, typename Epi, int UNR>
 __global__ void __launch_bounds__(kDirectThreads)
     k_sell_direct_packed(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+  stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
   using XB = typename std::conditional<std::is_same<V, __half>::value && std::is_same<X, __half>::value, __half,

@@ -693,6 +693,7 @@ __global__ void k_rich_scale_om(__half *__restrict__ hout, const RichState *__re
 __global__ void k_rich_axpy(__half *__restrict__ hout, const __half *__restrict__ t2,
                             const RichState *__restrict__ rs, int k, int use_ome, float *__restrict__ out,
                             __half *__restrict__ out16, float isc, int64_t n) {
+  stream_order();
   const float om = use_ome ? h2f(rs->ome[k]) : rs->om[k];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float hn = h2f(f2h(__fmaf_rn(om, h2f(t2[i]), h2f(hout[i]))));

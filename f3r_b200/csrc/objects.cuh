@@ -46,6 +46,9 @@ struct Context {
   double *pinned = nullptr;    // host-pinned scalars for D2H reads
   double *dscratch = nullptr;  // device scalars for f3r_dot
   int64_t launches = 0;        // kernels issued through this context
+  // launch_k lets a kernel be set up while its predecessor runs; set only while
+  // every kernel issued begins with stream_order()
+  bool overlap = false;
   std::vector<void *> allocs;
 
   Status alloc(void **p, size_t bytes) {
@@ -85,7 +88,21 @@ struct Context {
 template <typename... KP, typename... A>
 inline void launch_k(Context &c, void (*k)(KP...), dim3 grid, int block, size_t smem, cudaStream_t st,
                             A &&...args) {
-  k<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+  if (c.overlap) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, k, KP(std::forward<A>(args))...);  // the caller reads the launch error
+  } else {
+    k<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+  }
   c.launches++;
 }
 

@@ -167,6 +167,7 @@ template <typename V, typename X, typename Epi>
 __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
     k_sell_pattern(PatArgs A, const PatRun<V> *__restrict__ tab, const V *__restrict__ ival, const X *__restrict__ x,
                    Epi epi, int vec, int *err) {
+  stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
   using XB = typename std::conditional<std::is_same<V, __half>::value && std::is_same<X, __half>::value, __half,

@@ -1256,7 +1256,23 @@ template <int K> struct Engine {
 
   // What the outer level calls for one column: level 2, or (m2 = 0) the
   // fp16-vector level with its input and output through the slots.
-  Status outer_inner() { return p.m2 > 0 ? level2() : levelh(nullptr, nullptr, nullptr, nullptr); }
+  // Kernels of single-column solves are set up while their predecessors run
+  // (Context::overlap) where a launch is a good part of a kernel: systems of up to
+  // kOverlapRows rows, and short rows (many kernels of one wave after another).
+  // 16^3 27-point 1,531 -> 1,437 us, 40^3 2,461 -> 2,313, 7-point 50^3 3,162 ->
+  // 2,877, 90^3 10,609 -> 10,133.  Blocks of an early kernel go where room is left,
+  // which unbalances kernels sized for one even wave: 27-point 64^3 4,630 -> 4,912,
+  // row patterns at 100^3 8,418 -> 9,714, CSR at 40^3 2,644 -> 4,908; those launch
+  // in order.
+  static constexpr int32_t kOverlapRows = 1 << 16;
+  Status outer_inner() {
+    if (p.m2 <= 0) return levelh(nullptr, nullptr, nullptr, nullptr);
+    C().overlap = defer() && p.precond == F3R_PRECOND_SDAINV && !S.A.rptr &&
+                  (n <= kOverlapRows || S.A.max_width <= kDirectShort);
+    const Status s = level2();
+    C().overlap = false;
+    return s;
+  }
 
   // One call into level 2 for outer column j, replayed from a CUDA graph
   // keyed by which Richardson calls inside it update their weights.
