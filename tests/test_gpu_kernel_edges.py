@@ -119,3 +119,25 @@ def test_single_column_levels_are_the_block_kernels(ctx, grid, m2, m3):
         y = np.zeros(n)
         r = S.solve(B[k], y)
         assert r.is_solved and r.res_iter == rb[k].res_iter and np.array_equal(y, Y[k])
+
+
+@pytest.mark.parametrize("kw", [dict(aligned=True), dict(aligned=True, height=64)])
+def test_patterns_and_streamed_kernels_agree_on_non_finite_x(ctx, kw):
+    """infinities and NaN in x reach the same rows from the row patterns as from
+    the streamed kernel (which x off a 16-byte boundary takes), through padding
+    and absent entries too"""
+    A = F.stencil27(83, 71, 53, 2, 0.5).scale()
+    n = A.shape[0]
+    S = F.Sell(ctx, A, **kw)
+    x = np.random.default_rng(5).standard_normal(n)
+    x[[0, 1, 40, n // 2, n - 1]] = [np.inf, np.nan, -np.inf, np.inf, np.nan]
+    for vt, tdt in ((F.F64, torch.float64), (F.F32, torch.float32), (F.F16, torch.float32), (F.F16, torch.float16)):
+        xa = torch.from_numpy(x).to(tdt).cuda()
+        xo = torch.zeros(n + 1, dtype=tdt, device="cuda")[1:]
+        xo.copy_(xa)
+        ya, yo = torch.zeros_like(xa), torch.zeros_like(xa)
+        S.operate(xa, ya, val_t=vt)
+        S.operate(xo, yo, val_t=vt)
+        torch.cuda.synchronize()
+        assert np.array_equal(ya.cpu().numpy(), yo.cpu().numpy(), equal_nan=True), vt
+    S.close()
