@@ -31,7 +31,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, K * sizeof(typename acc_
   PatRun<V> *pats = reinterpret_cast<PatRun<V> *>(psm + (size_t)A.stages * A.elems * RB);
   __shared__ uint64_t full[kPatStages], empty[kPatStages];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t nfl = (int64_t)A.n / PER * PER;
+  const int64_t nfl = (int64_t)A.ncols / PER * PER;
   if (threadIdx.x == 0) {
     for (int s = 0; s < A.stages; s++) {
       mbar_init(&full[s], 1);
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, K * sizeof(typename acc_
     if (PER > 1 && t >= A.tail_tile) {  // x's last rows, short of a 16-byte unit
       for (int w = 0; w < A.nwin; w++) {
         const int64_t a = r0 + A.win[w].lo, i = nfl + lane;
-        if (i < A.n && i >= a && i < a + A.win[w].len) {
+        if (i < A.ncols && i >= a && i < a + A.win[w].len) {
 #pragma unroll
           for (int c = 0; c < K; c++) sx[(A.win[w].base + (i - a)) * K + c] = x[i * K + c];
         }

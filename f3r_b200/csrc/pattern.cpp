@@ -289,6 +289,7 @@ static bool layout(const SellHost &h, int sm_count, Layout &o) {
   // tiles of 2,048 rows, half of that on smaller systems so that every SM gets several
   o.warps = n >= (int64_t)sm_count * 4096 ? kPatWarps : kPatWarps / 2;
   a.n = (int32_t)n;
+  a.ncols = h.ncols;
   a.nblk = nblk;
   a.tile = o.warps * kPatBlock;
   a.ntiles = (int32_t)cdiv(n, a.tile);

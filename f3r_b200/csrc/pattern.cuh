@@ -58,7 +58,8 @@ struct PatWindow {
 };
 
 struct PatArgs {
-  int32_t n, nblk, ntiles, tile;         // rows, 128-row blocks, tiles, rows a tile
+  int32_t n, nblk, ntiles, tile;         // rows, 256-row blocks, tiles, rows a tile
+  int32_t ncols;                         // columns: the elements of x, what copies and columns stay below
   int32_t np, stride, nwin, elems;       // patterns, records a pattern, windows, elements of a stage
   int32_t stages, tail_tile;             // tiles from tail_tile on reach x's last, partial 16-byte unit
   PatWindow win[kPatWindows];
@@ -160,7 +161,7 @@ template <typename E> inline bool epi_vec4(const E &e) {
 }
 
 // blockDim.x = (warps + 1) * 32: `warps` warps work a tile of warps * kPatBlock
-// rows, each its 128, and never wait for one another; the last warp's first
+// rows, each its block, and never wait for one another; the last warp's first
 // lane keeps the windows of the next tiles coming (a full and an empty mbarrier
 // a stage, every wait bounded).
 template <typename V, typename X, typename Epi>
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
   PatRun<V> *pats = reinterpret_cast<PatRun<V> *>(psm + (size_t)A.stages * A.elems * sizeof(X));
   __shared__ uint64_t full[kPatStages], empty[kPatStages];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x >> 5) - 1;
-  const int64_t nfl = (int64_t)A.n / (16 / (int)sizeof(X)) * (16 / (int)sizeof(X));  // what bulk copies can bring
+  const int64_t nfl = (int64_t)A.ncols / (16 / (int)sizeof(X)) * (16 / (int)sizeof(X));  // what bulk copies can bring
   if (threadIdx.x == 0) {
     for (int s = 0; s < A.stages; s++) {
       mbar_init(&full[s], 1);
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
       // x's last elements, short of a 16-byte unit: every warp that may read them writes them (the same values)
       for (int w = 0; w < A.nwin; w++) {
         const int64_t a = r0 + A.win[w].lo, i = nfl + lane;
-        if (i < A.n && i >= a && i < a + A.win[w].len) sx[A.win[w].base + (i - a)] = x[i];
+        if (i < A.ncols && i >= a && i < a + A.win[w].len) sx[A.win[w].base + (i - a)] = x[i];
       }
       __syncwarp();
     }
@@ -389,12 +390,12 @@ struct PatShape {
 inline int64_t pattern_rows(int sm_count, int height, size_t sv) {
   return (int64_t)sm_count * (height == 64 && sv == 2 ? 2048 : 1024);
 }
-// the first tile whose windows pass the last of n rows that whole units of `per` rows bring
+// the first tile whose windows pass the last of x that whole units of `per` elements bring
 inline int32_t pattern_tail(const PatArgs &a, int64_t per) {
   int64_t hi = 0;
   for (int w = 0; w < a.nwin; w++) hi = std::max<int64_t>(hi, (int64_t)a.win[w].lo + a.win[w].len);
-  const int64_t nfl = a.n / per * per;
-  return nfl == a.n ? a.ntiles : (int32_t)std::max<int64_t>(0, (nfl - hi) / a.tile);
+  const int64_t nfl = a.ncols / per * per;
+  return nfl == a.ncols ? a.ntiles : (int32_t)std::max<int64_t>(0, (nfl - hi) / a.tile);
 }
 inline PatShape pattern_shape(const PatArgs &a, int warps, size_t sx, size_t st) {
   const size_t one = (size_t)a.elems * sx, table = (size_t)a.np * a.stride * st, sm = 227 * 1024;

@@ -81,6 +81,35 @@ def test_products_bitexact_across_the_rules(ctx, kind, grid, kw):
     S.close()
 
 
+@pytest.mark.parametrize("height", [32, 64])
+@pytest.mark.parametrize("nrows,ncols,offsets", [
+    (310007, 310033, tuple(range(27))),                                          # more columns than rows
+    (310007, 309006, (-1300, -1299, -1298, -40, -39, -38) + tuple(range(-3, 6))),  # fewer
+    (310007, 620013, (0, 1, 2, 5, 6, 7, 155000, 155001, 155002, 310003, 310004, 310005)),  # a window past the rows
+])
+def test_products_of_rectangular_matrices_with_repeating_rows(ctx, height, nrows, ncols, offsets):
+    """bands of constant coefficients whose columns do not end where the rows do: the oracle's sums bit for bit"""
+    d = np.array(offsets)
+    c = np.arange(nrows)[:, None] + d
+    keep = (c >= 0) & (c < ncols)
+    r = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    i = c[keep].astype(np.int32)
+    v = np.broadcast_to(np.random.default_rng(8).standard_normal(len(d)), c.shape)[keep]
+    S = F.Sell(ctx, F.HostMatrix.from_csr(r, i, v, ncols), aligned=True, height=height)
+    x = np.random.default_rng(9).standard_normal(ncols)
+    for vt, dt, tdt, ov, oy, oacc in ((F.F64, np.float64, torch.float64, O.DT_F64, O.DT_F64, O.DT_F64),
+                                      (F.F32, np.float32, torch.float32, O.DT_F32, O.DT_F32, O.DT_F32),
+                                      (F.F16, np.float32, torch.float32, O.DT_F16, O.DT_F32, O.DT_F32),
+                                      (F.F16, np.float16, torch.float16, O.DT_F16, O.DT_F16, O.DT_F32)):
+        xd = x.astype(dt)
+        y = torch.zeros(nrows, dtype=tdt, device="cuda")
+        S.operate(torch.from_numpy(xd).cuda(), y, val_t=vt)
+        torch.cuda.synchronize()
+        want = O.spmv(r, i, v, xd, ov, oy, oacc)
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
+    S.close()
+
+
 @pytest.mark.parametrize("n,lo,hi", [(1, 1, 1), (97, 0, 8), (64, 8, 8), (131, 9, 9), (70, 30, 70), (33, 0, 33)])
 def test_csr_tiles_bitexact(ctx, n, lo, hi):
     """groups of 32 rows that fit the short tile, fill it, fit the wide one or
