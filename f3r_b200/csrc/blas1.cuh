@@ -116,7 +116,7 @@ __device__ __forceinline__ float final_sums1(const float *part, int lgrid, int q
 // H(j, k) = <w, V(k)>, k < nv <= NV, all with the unmodified w (gmres.hpp:112-114)
 template <int NV, int L>
 __global__ void __launch_bounds__(256, 4)
-    k_dots1(const float *__restrict__ w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, float *__restrict__ hcol) {
+    k_dots1(const float *w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, float *hcol) {
   stream_order();
   __shared__ float sred[8][L * NV];
   __shared__ float sw[8][4];
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256, 4)
   float a[L][NV], sc[NV];
 #pragma unroll
   for (int k = 0; k < NV; k++) {
-    sc[k] = k < nv && V.s[k] ? __ldg(V.s[k]) : 1.0f;
+    sc[k] = k < nv && V.s[k] ? *V.s[k] : 1.0f;
 #pragma unroll
     for (int l = 0; l < L; l++) a[l][k] = 0.0f;
   }
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
     for (int l = 0; l < L; l++)
       if (l == 0 || (q + l * 256 < nq && blockIdx.x * L + l < lgrid)) {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(w) + q + l * 256);
+        const float4 t = ld_stream(reinterpret_cast<const float4 *>(w) + q + l * 256);
         wv[l][0] = t.x; wv[l][1] = t.y; wv[l][2] = t.z; wv[l][3] = t.w;
       }
 #pragma unroll
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
           for (int l = 0; l < L; l++)
             if (l == 0 || (q + l * 256 < nq && blockIdx.x * L + l < lgrid))
-              v[k][l] = __ldg(reinterpret_cast<const float4 *>(V.p[k0 + k]) + q + l * 256);
+              v[k][l] = ld_stream(reinterpret_cast<const float4 *>(V.p[k0 + k]) + q + l * 256);
         }
 #pragma unroll
       for (int k = 0; k < 4; k++)
@@ -239,7 +239,7 @@ struct Givens8 {
 // Givens rotation and, on the level's last step, y (gmres.hpp:115-121); nv = j + 1 <= 8
 template <int NV, int L>
 __global__ void __launch_bounds__(256, 4)
-    k_cgs1(float *__restrict__ w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, LevelK<float> Lv, int j,
+    k_cgs1(float *w, Basis8 V, int nv, int64_t n, int lgrid, GridRed gr, LevelK<float> Lv, int j,
            int compute_y, int *err) {
   stream_order();
   __shared__ float sh[kMaxDots1], ssc[kMaxDots1];
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256, 4)
         if (k0 + k < nv) {
 #pragma unroll
           for (int l = 0; l < L; l++)
-            if (live(l)) v[k][l] = __ldg(reinterpret_cast<const float4 *>(V.p[k0 + k]) + q + l * 256);
+            if (live(l)) v[k][l] = ld_stream(reinterpret_cast<const float4 *>(V.p[k0 + k]) + q + l * 256);
         }
 #pragma unroll
       for (int k = 0; k < 4; k++)
@@ -325,8 +325,8 @@ __global__ void __launch_bounds__(256, 4)
 
 // x = Z y of level 3 from its fp16 basis (gmres.hpp:127-128): 8 rows a thread,
 // nz <= 8 columns, widened exactly, MULMV order
-__global__ void __launch_bounds__(256) k_zy1(const __half *__restrict__ Z, int64_t ldz, const float *__restrict__ y, int nz,
-                                             float *__restrict__ out, int64_t n) {
+__global__ void __launch_bounds__(256) k_zy1(const __half *Z, int64_t ldz, const float *y, int nz, float *out,
+                                             int64_t n) {
   stream_order();
   __shared__ float sy[kMaxDots1];
   if ((int)threadIdx.x < nz) sy[threadIdx.x] = y[threadIdx.x];
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(256) k_zy1(const __half *__restrict__ Z, int64
       uint4 u[4];
 #pragma unroll
       for (int k = 0; k < 4; k++)
-        if (k0 + k < nz) u[k] = __ldg(reinterpret_cast<const uint4 *>(Z + (k0 + k) * ldz + i0));
+        if (k0 + k < nz) u[k] = ld_stream(reinterpret_cast<const uint4 *>(Z + (k0 + k) * ldz + i0));
 #pragma unroll
       for (int k = 0; k < 4; k++)
         if (k0 + k < nz) {

@@ -994,8 +994,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_resnormK(const double *__restric
 // running mean ome[k] = fp16(sum[k] / den); k = 0 also advances den.  Rows
 // in groups of 4 per thread, block-strided final stage.
 template <int WARPS, int K>
-__global__ void __launch_bounds__(WARPS * 32) k_rich_weightK(const __half *__restrict__ tmp,
-                                                             const __half *__restrict__ other, int64_t n,
+__global__ void __launch_bounds__(WARPS * 32) k_rich_weightK(const __half *tmp,
+                                                             const __half *other, int64_t n,
                                                              GridRed gr, RichState *rs, int k) {
   stream_order();
   __shared__ float sred[WARPS][2 * K];
@@ -1059,8 +1059,8 @@ template <int R, typename F> __device__ __forceinline__ void for_row_groups(int6
 // Level-2 entry (k_level2_enter): V1(j)(:, c) *= 1/h_c in place, then
 // V2(0) = float(V1(j)); e_c(0) = 1.
 template <int K>
-__global__ void k_level2_enterK(double *const *__restrict__ in_slot, const double *__restrict__ inv,
-                                float *__restrict__ v0, float *e, int64_t e_stride, int64_t n) {
+__global__ void k_level2_enterK(double *const *in_slot, const double *inv,
+                                float *v0, float *e, int64_t e_stride, int64_t n) {
   stream_order();
   double *in = *in_slot;
   double s[K];
@@ -1085,7 +1085,7 @@ __global__ void k_level2_enterK(double *const *__restrict__ in_slot, const doubl
 // x(:, c) = Z y_c (inner levels) or x(:, c) += Z y_c for the columns in mask
 // (outer level), the sum in the level's type T (k_zy)
 template <typename T, typename Out, bool ACCUM, int K, typename ZT = T>
-__global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_zyK(Cols<ZT> Z, const T *__restrict__ y, int64_t y_stride, int nz, Out *out_direct,
+__global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_zyK(Cols<ZT> Z, const T *y, int64_t y_stride, int nz, Out *out_direct,
                       Out *const *out_slot, uint32_t mask, int64_t n) {
   stream_order();
   __shared__ T sy[K][kMaxCols];
@@ -1125,9 +1125,9 @@ __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_zyK(Cols<ZT> Z, 
 // hout = M hin, times ome_c[0] on a call without a weight update; e_c(0) = 1
 // of the calling level when e_set is given.
 template <bool SCALE_BY_OME, int K, int NR, bool MM>
-__device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ in, bool normalise, bool store, const float (&s)[K],
+__device__ __forceinline__ void rich_enter_rows(int64_t i0, float *in, bool normalise, bool store, const float (&s)[K],
                                                 const float (&om)[K], float sc, const DiagPre &M,
-                                                __half *__restrict__ hin, __half *__restrict__ hout) {
+                                                __half *hin, __half *hout) {
   constexpr int E = NR * K, NM = MM ? E : NR;  // diagonal values: per row, or per row and column
   float v[E], w[NM], z[NM];
   __half hi[E], ho[E];
@@ -1152,9 +1152,9 @@ __device__ __forceinline__ void rich_enter_rows(int64_t i0, float *__restrict__ 
 }
 
 template <bool SCALE_BY_OME, int K, bool MM = false>
-__global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK(float *__restrict__ in, const float *__restrict__ in_inv, float sc, DiagPre M,
-                                   __half *__restrict__ hin, __half *__restrict__ hout,
-                                   const RichState *__restrict__ rs, float *e_set, int64_t e_stride, int64_t n, bool store) {
+__global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK(float *in, const float *in_inv, float sc, DiagPre M,
+                                   __half *hin, __half *hout,
+                                   const RichState *rs, float *e_set, int64_t e_stride, int64_t n, bool store) {
   stream_order();
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   float om[K], s[K];
@@ -1175,8 +1175,8 @@ __global__ void __launch_bounds__(kEwThreads, K == 1 ? 8 : 1) k_rich_enter_diagK
 
 // General M: (normalise, in place where store), hin = fp16(in * sc) (k_rich_cast_in)
 template <int K>
-__global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict__ in_inv, float sc,
-                                __half *__restrict__ hin, float *e_set, int64_t e_stride, int64_t n, bool store) {
+__global__ void k_rich_cast_inK(float *in, const float *in_inv, float sc,
+                                __half *hin, float *e_set, int64_t e_stride, int64_t n, bool store) {
   stream_order();
   if (e_set && blockIdx.x == 0 && threadIdx.x < K) e_set[threadIdx.x * e_stride] = 1.0f;
   for_row_groups<RowsPer<K>::R>(n, [&](int64_t i0, auto rows) {
@@ -1196,7 +1196,7 @@ __global__ void k_rich_cast_inK(float *__restrict__ in, const float *__restrict_
 
 // hout(:, c) = fp16(hout * fp16(om_c[0])) (k_rich_scale_om)
 template <int K>
-__global__ void k_rich_scale_omK(__half *__restrict__ hout, const RichState *__restrict__ rs, int64_t n) {
+__global__ void k_rich_scale_omK(__half *hout, const RichState *rs, int64_t n) {
   stream_order();
   float om[K];
 #pragma unroll
@@ -1214,9 +1214,9 @@ __global__ void k_rich_scale_omK(__half *__restrict__ hout, const RichState *__r
 // hout(:, c) = fp16(hout + om_c[k] t2), or on the last step out = fp32(that)
 // / sc (k_rich_axpy); use_ome selects ome_c[k]
 template <int K>
-__global__ void k_rich_axpyK(__half *__restrict__ hout, const __half *__restrict__ t2,
-                             const RichState *__restrict__ rs, int k, int use_ome, float *__restrict__ out, float isc,
-                             int64_t n, __half *__restrict__ out16) {
+__global__ void k_rich_axpyK(__half *hout, const __half *t2,
+                             const RichState *rs, int k, int use_ome, float *out, float isc,
+                             int64_t n, __half *out16) {
   stream_order();
   float om[K];
 #pragma unroll
@@ -1240,7 +1240,7 @@ __global__ void k_rich_axpyK(__half *__restrict__ hout, const __half *__restrict
 
 // out = fp32(hout) / sc (k_rich_exit)
 template <int K>
-__global__ void k_rich_exitK(const __half *__restrict__ hout, float *__restrict__ out, float isc, int64_t n) {
+__global__ void k_rich_exitK(const __half *hout, float *out, float isc, int64_t n) {
   stream_order();
   for_row_groups<RowsPer<K>::R>(n, [&](int64_t i0, auto rows) {
     constexpr int E = decltype(rows)::value * K;

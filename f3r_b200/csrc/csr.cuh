@@ -39,7 +39,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 
 template <typename V, typename X, typename Epi, int T>
 __global__ void __launch_bounds__(kCsrWarps * 32)
-    k_csr_group(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+    k_csr_group(const V *__restrict__ val, DevSell A, const X *x, Epi epi) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kCsrWarps * 32)
       Acc xv[B];
 #pragma unroll
       for (int e = 0; e < B; e++)
-        if (k + e < hi) xv[e] = to_acc<Acc>(__ldg(x + sc[k + e]));
+        if (k + e < hi) xv[e] = to_acc<Acc>(ld_stream(x + sc[k + e]));
 #pragma unroll
       for (int e = 0; e < B; e++)
         if (k + e < hi) acc = fmaT(to_acc<Acc>(sv[k + e]), xv[e], acc);

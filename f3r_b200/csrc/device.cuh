@@ -81,11 +81,37 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 // Start of a kernel that may be launched while its predecessor still runs
 // (Context::overlap): waits until the predecessor has finished and its writes are
 // visible, then lets the successor be launched.  Nothing before it may touch
-// memory that another kernel of the stream writes or reads.  No effect in an
-// ordinary launch.
+// memory that another kernel of the stream writes or reads.  What such a kernel
+// reads of other kernels' results it reads by ld_stream, or by plain loads through
+// pointers without __restrict__: read-only loads (__ldg, or what a compiler makes
+// of const __restrict__) are defined only where nothing writes the data during the
+// kernel's life, which now begins before its predecessor ends, and may be moved
+// above the wait.  No effect in an ordinary launch.
 __device__ __forceinline__ void stream_order() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// A coherent load of 2, 4, 8 or 16 bytes that stays behind stream_order() (volatile,
+// as the wait is) and leaves the other memory accesses free to be moved.
+template <typename T> __device__ __forceinline__ T ld_stream(const T *p) {
+  static_assert(sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "ld_stream");
+  if constexpr (sizeof(T) == 2) {
+    unsigned short u;
+    asm volatile("ld.global.b16 %0, [%1];" : "=h"(u) : "l"(p));
+    return *reinterpret_cast<const T *>(&u);
+  } else if constexpr (sizeof(T) == 4) {
+    uint32_t u;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(u) : "l"(p));
+    return *reinterpret_cast<const T *>(&u);
+  } else if constexpr (sizeof(T) == 8) {
+    uint64_t u;
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(u) : "l"(p));
+    return *reinterpret_cast<const T *>(&u);
+  } else {
+    uint4 u;
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p));
+    return *reinterpret_cast<const T *>(&u);
+  }
 }
 // L2 policy for streamed-once data (matrix values and indices): evict first,
 // so the gathered vector stays resident in L2.

@@ -98,7 +98,7 @@ __device__ __forceinline__ void direct_aligned_rows(const V *val, const DevSell 
       for (int e = 0; e < W; e++) {
         int32_t c = b[k][e] + q;
         if (cp[k] & 1) c = min(max(c, 0), A.ncols - 1);
-        xg[i][e] = to_acc<XB>(__ldg(x + c));
+        xg[i][e] = to_acc<XB>(ld_stream(x + c));
       }
     }
   }
@@ -112,7 +112,7 @@ __device__ __forceinline__ void direct_aligned_rows(const V *val, const DevSell 
 // 32 R w ... , R a lane
 template <typename V, typename X, typename Epi, int H, int R>
 __global__ void __launch_bounds__(kDirectThreads)
-    k_sell_direct_aligned(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+    k_sell_direct_aligned(const V *__restrict__ val, DevSell A, const X *x, Epi epi) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kDirectThreads)
 // or with explicit columns among them (the mixed form); a row a lane
 template <typename V, typename X, typename Epi, int H>
 __global__ void __launch_bounds__(kDirectThreads)
-    k_sell_direct_mixed(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+    k_sell_direct_mixed(const V *__restrict__ val, DevSell A, const X *x, Epi epi) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kDirectThreads)
       for (int e = 0; e < W; e++) c[e] = __ldg(A.col + (size_t)xo + e * 32 + q);
     }
 #pragma unroll
-    for (int e = 0; e < W; e++) xg[e] = to_acc<XB>(__ldg(x + c[e]));
+    for (int e = 0; e < W; e++) xg[e] = to_acc<XB>(ld_stream(x + c[e]));
 #pragma unroll
     for (int e = 0; e < W; e++) acc = fma_vx<Acc>(v[e], xg[e], acc);
   };
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kDirectThreads)
 // Packed int32 slices, UNR columns at a time
 template <typename V, typename X, typename Epi, int UNR>
 __global__ void __launch_bounds__(kDirectThreads)
-    k_sell_direct_packed(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi) {
+    k_sell_direct_packed(const V *__restrict__ val, DevSell A, const X *x, Epi epi) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kDirectThreads)
       }
 #pragma unroll
     for (int e = 0; e < UNR; e++)
-      if (full || k0 + e < w) xg[e] = to_acc<XB>(__ldg(x + c[e]));
+      if (full || k0 + e < w) xg[e] = to_acc<XB>(ld_stream(x + c[e]));
 #pragma unroll
     for (int e = 0; e < UNR; e++)
       if (full || k0 + e < w) acc = fma_vx<Acc>(v[e], xg[e], acc);

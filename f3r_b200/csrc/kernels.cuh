@@ -690,9 +690,9 @@ __global__ void k_rich_scale_om(__half *__restrict__ hout, const RichState *__re
 // hout = fp16(hout + om[k] t2) (f3r-gpu.cpp:252), or on the last step out =
 // fp32(that) / sc, or out16 = that (R below the fp16-vector level).  use_ome
 // selects ome[k] (no-update calls, general M).
-__global__ void k_rich_axpy(__half *__restrict__ hout, const __half *__restrict__ t2,
-                            const RichState *__restrict__ rs, int k, int use_ome, float *__restrict__ out,
-                            __half *__restrict__ out16, float isc, int64_t n) {
+__global__ void k_rich_axpy(__half *hout, const __half *t2,
+                            const RichState *rs, int k, int use_ome, float *out,
+                            __half *out16, float isc, int64_t n) {
   stream_order();
   const float om = use_ome ? h2f(rs->ome[k]) : rs->om[k];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {

@@ -166,7 +166,7 @@ template <typename E> inline bool epi_vec4(const E &e) {
 // a stage, every wait bounded).
 template <typename V, typename X, typename Epi>
 __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
-    k_sell_pattern(PatArgs A, const PatRun<V> *__restrict__ tab, const V *__restrict__ ival, const X *__restrict__ x,
+    k_sell_pattern(PatArgs A, const PatRun<V> *__restrict__ tab, const V *__restrict__ ival, const X *x,
                    Epi epi, int vec, int *err) {
   stream_order();
   epi_setup(epi, 0);
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
       V u[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        xg[e] = to_acc<XB>(__ldg(x + c[e]));
+        xg[e] = to_acc<XB>(ld_stream(x + c[e]));
         u[e] = v[e];
       }
       if (k + 4 < w) entries(k + 4);

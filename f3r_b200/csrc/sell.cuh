@@ -149,7 +149,7 @@ constexpr size_t sell_smem_bytes() {
 // (cbase for aligned slices, col from xoff for the others) or AllAlignedIdx.
 template <typename V, typename X, typename Epi, int WARPS, int STAGES, int KC, typename CI = int32_t>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-    k_sell_cfg(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi, int *err) {
+    k_sell_cfg(const V *__restrict__ val, DevSell A, const X *x, Epi epi, int *err) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -293,10 +293,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
             for (int e = 0; e < 4; e++) v[g * 4 + e] = t[e];
             if (!clampc) {
 #pragma unroll
-              for (int e = 0; e < 4; e++) xg[g * 4 + e] = to_acc<XB>(__ldg(xl + b[e]));
+              for (int e = 0; e < 4; e++) xg[g * 4 + e] = to_acc<XB>(ld_stream(xl + b[e]));
             } else {
 #pragma unroll
-              for (int e = 0; e < 4; e++) xg[g * 4 + e] = to_acc<XB>(__ldg(x + min(max(b[e] + lane, 0), A.ncols - 1)));
+              for (int e = 0; e < 4; e++) xg[g * 4 + e] = to_acc<XB>(ld_stream(x + min(max(b[e] + lane, 0), A.ncols - 1)));
             }
           }
         }
@@ -365,13 +365,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
       XB xv[KC];
       if (full) {
 #pragma unroll
-        for (int k = 0; k < KC; k++) xv[k] = to_acc<XB>(__ldg(x + cc[k]));
+        for (int k = 0; k < KC; k++) xv[k] = to_acc<XB>(ld_stream(x + cc[k]));
 #pragma unroll
         for (int k = 0; k < KC; k++) acc = fma_vx<Acc>(vv[k], xv[k], acc);
       } else {
 #pragma unroll
         for (int k = 0; k < KC; k++)
-          if (k < kc) xv[k] = to_acc<XB>(__ldg(x + cc[k]));
+          if (k < kc) xv[k] = to_acc<XB>(ld_stream(x + cc[k]));
 #pragma unroll
         for (int k = 0; k < KC; k++)
           if (k < kc) acc = fma_vx<Acc>(vv[k], xv[k], acc);
@@ -432,7 +432,7 @@ static_assert(sell64_smem_bytes<__half>() <= 227 * 1024 && sell64_smem_bytes<flo
 
 template <typename V, typename X, typename Epi, int WARPS, int STAGES, int KC>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-    k_sell64(const V *__restrict__ val, DevSell A, const X *__restrict__ x, Epi epi, int *err) {
+    k_sell64(const V *__restrict__ val, DevSell A, const X *x, Epi epi, int *err) {
   stream_order();
   epi_setup(epi, 0);
   using Acc = typename acc_of<V>::type;
@@ -562,14 +562,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
               const X *px = xl + b[e];
-              g0[g * 4 + e] = to_acc<XB>(__ldg(px));
-              g1[g * 4 + e] = to_acc<XB>(__ldg(px + 32));
+              g0[g * 4 + e] = to_acc<XB>(ld_stream(px));
+              g1[g * 4 + e] = to_acc<XB>(ld_stream(px + 32));
             }
           } else {
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-              g0[g * 4 + e] = to_acc<XB>(__ldg(x + min(max(b[e] + lane, 0), A.ncols - 1)));
-              g1[g * 4 + e] = to_acc<XB>(__ldg(x + min(max(b[e] + lane + 32, 0), A.ncols - 1)));
+              g0[g * 4 + e] = to_acc<XB>(ld_stream(x + min(max(b[e] + lane, 0), A.ncols - 1)));
+              g1[g * 4 + e] = to_acc<XB>(ld_stream(x + min(max(b[e] + lane + 32, 0), A.ncols - 1)));
             }
           }
         }
