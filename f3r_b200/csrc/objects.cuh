@@ -209,8 +209,10 @@ inline bool launch_pattern(Context &c, const V *val, const DevPattern &d, const 
   a.stages = p.stages;
   a.tail_tile = pattern_tail(a, 16 / (int64_t)sizeof(X));
   const int64_t work = std::max<int64_t>(a.ntiles, cdiv(a.ngroups, d.warps));
-  launch_k(c, k_sell_pattern<V, X, Epi>, (unsigned)std::min<int64_t>(work, (int64_t)c.sm_count * p.ctas), (d.warps + 1) * 32,
-           p.smem, c.stream, a, d.tab(val), d.vals(val), x, epi, epi_vec4(epi) ? 1 : 0, c.err);
+  const int grid = (int)std::min<int64_t>(work, (int64_t)c.sm_count * p.ctas);
+  a.rest = PatRest(a.ntiles, a.ngroups, d.warps, grid);
+  launch_k(c, k_sell_pattern<V, X, Epi>, (unsigned)grid, (d.warps + 1) * 32, p.smem, c.stream, a, d.tab(val),
+           d.vals(val), x, epi, epi_vec4(epi) ? 1 : 0, c.err);
   return true;
 }
 

@@ -68,8 +68,9 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, K * sizeof(typename acc_
     for (int k = max(0, i - A.stages); k < i; k++) mbar_wait_bounded(&full[k % A.stages], (uint32_t)(k / A.stages) & 1u);
     return;
   }
-  const int busy = A.ntiles % (int)gridDim.x, idle = (int)gridDim.x - busy;
-  for (int g = ((int)blockIdx.x - busy) * kPatWarps + warp; g >= 0 && g < A.ngroups; g += idle * kPatWarps) {
+  for (int q = A.rest.begin(blockIdx.x, gridDim.x); q < A.rest.rounds; q = A.rest.next(q, blockIdx.x, gridDim.x)) {
+    const int g = q * kPatWarps + warp;
+    if (g >= A.ngroups) break;
     const int32_t r = A.irow[(size_t)g * 32 + lane], k0 = A.iptr[g], w = A.iptr[g + 1] - k0;
     if (r < 0) continue;
     const int32_t *lc = A.icol + (size_t)k0 * 32 + lane;

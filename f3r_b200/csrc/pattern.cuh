@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "patrest.hpp"
 #include "sell.cuh"
 
 namespace f3r {
@@ -66,6 +67,7 @@ struct PatArgs {
   const uint8_t *blk;                    // per block: its pattern
   const uint8_t *live;                   // per block and lane: which of its 8 rows follow it (4 of each half)
   int32_t ngroups;                       // the other rows, 32 a group
+  PatRest rest;                          // who works them
   const int32_t *irow, *iptr, *icol;     // row (-1: none); first entry / 32 (ngroups + 1); columns, entry k of lane l at k * 32 + l
 };
 
@@ -217,10 +219,10 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
     return;
   }
   typename Epi::Red none[1];
-  // the rows off their block's pattern, while the first windows arrive; the
-  // CTAs with a tile fewer than the first ones take them
-  const int busy = A.ntiles % (int)gridDim.x, idle = (int)gridDim.x - busy;
-  for (int g = ((int)blockIdx.x - busy) * warps + warp; g >= 0 && g < A.ngroups; g += idle * warps) {
+  // the rows off their block's pattern, while the first windows arrive
+  for (int q = A.rest.begin(blockIdx.x, gridDim.x); q < A.rest.rounds; q = A.rest.next(q, blockIdx.x, gridDim.x)) {
+    const int g = q * warps + warp;
+    if (g >= A.ngroups) break;
     const int32_t r = A.irow[(size_t)g * 32 + lane], k0 = A.iptr[g], w = A.iptr[g + 1] - k0;
     if (r < 0) continue;
     const int32_t *lc = A.icol + (size_t)k0 * 32 + lane;

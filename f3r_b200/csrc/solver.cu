@@ -696,8 +696,9 @@ bool launch_pattern_block(Context &c, const V *val, const DevPattern &d, const X
   a.stages = p.stages;
   a.tail_tile = pattern_tail(a, std::max<int64_t>(1, 16 / (int64_t)(sizeof(X) * K)));
   const int64_t work = std::max<int64_t>(a.ntiles, cdiv(a.ngroups, kPatWarps));
-  launch_k(c, k_pattern_block<V, X, Epi, K>, (unsigned)std::min<int64_t>(work, (int64_t)c.sm_count * std::min(p.ctas, 3)),
-           (kPatWarps + 1) * 32, p.smem, c.stream, a, d.tab(val, 1), d.vals(val), x, epi, c.err);
+  const int grid = (int)std::min<int64_t>(work, (int64_t)c.sm_count * std::min(p.ctas, 3));
+  a.rest = PatRest(a.ntiles, a.ngroups, kPatWarps, grid);
+  launch_k(c, k_pattern_block<V, X, Epi, K>, (unsigned)grid, (kPatWarps + 1) * 32, p.smem, c.stream, a, d.tab(val, 1), d.vals(val), x, epi, c.err);
   return true;
 }
 template <typename V, typename X, typename Epi, int K>

@@ -49,6 +49,7 @@ def test_block_ilu_solve_is_the_oracles(ctx, grid, blocks, sigma):
     # repeating rows (from half a wave of rows, or a wave): one and three windows, ragged grids, both tile sizes
     ("27pt", (40, 31, 17), dict(aligned=True, height=64)), ("27pt", (54, 53, 53), dict(aligned=True)),
     ("27pt", (200, 3, 261), dict(aligned=True)), ("27pt", (101, 67, 59), dict(aligned=True, height=64)),
+    ("27pt", (107, 106, 106), dict(aligned=True)),  # rows off the patterns beside a last wave of tiles that is nearly full
     ("27pt", (81, 81, 81), dict(aligned=True)), ("27pt", (97, 90, 81), dict(aligned=True, height=64)),
     ("27pt", (53, 53, 53), dict(sigma=256)), ("27pt", (54, 53, 53), dict(sigma=256)),  # and of half of one (fp64)
 ])

@@ -1,6 +1,7 @@
 """Rules on the kernels' sources that no run can show broken."""
 import os
 import re
+import subprocess
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "f3r_b200", "csrc")
 # what no kernel of a stream writes: a matrix's values, columns, slot bases and row patterns
@@ -29,3 +30,39 @@ def test_kernels_that_may_start_early_read_results_coherently():
             for a in re.findall(r"__ldg\((.*)", s):
                 assert CONSTANT.match(a), (f, a)
     assert kernels >= 15
+
+
+def test_rows_off_the_patterns_are_dealt_evenly(tmp_path):
+    """every round to one CTA, and no CTA with more than its share of tiles and
+    rounds (a tile as kRestSpare rounds) and one of each, whatever the last wave holds"""
+    src = tmp_path / "rest.cpp"
+    src.write_text(r'''
+#include <cstdio>
+#include <vector>
+#include "patrest.hpp"
+using namespace f3r;
+int main() {
+  for (int grid : {1, 2, 147, 148, 296, 444, 592})
+    for (int tiles : {0, 1, 146, 147, 148, 295, 442, 443, 444, 583, 1175, 2662, 3456})
+      for (int groups : {0, 1, 7, 8, 9, 985, 2058, 4000, 16815, 400000}) {
+        const PatRest r(tiles, groups, 8, grid);
+        std::vector<int> seen(r.rounds, 0);
+        const double share = (tiles * (double)kRestSpare + r.rounds) / grid;
+        for (int c = 0; c < grid; c++) {
+          int mine = 0;
+          for (int q = r.begin(c, grid); q < r.rounds; q = r.next(q, c, grid), mine++) seen[q]++;
+          const int t = c < tiles ? (tiles - 1 - c) / grid + 1 : 0;
+          const double load = t * (double)kRestSpare + mine;
+          if (mine && load > share + kRestSpare + 1) return std::printf("%d %d %d: CTA %d %d + %d\\n", grid, tiles, groups, c, t, mine), 1;
+        }
+        for (int k : seen)
+          if (k != 1) return std::printf("%d %d %d: a round dealt %d times\\n", grid, tiles, groups, k), 1;
+        if (r.rounds * 8 < groups || (r.rounds - 1) * 8 >= groups + 8) return 1;
+      }
+  return 0;
+}
+''')
+    exe = tmp_path / "rest"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
