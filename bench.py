@@ -241,12 +241,12 @@ def spmv_roofline(solver, A, torch, F):
     algorithmic bytes, nnz * (2 + 4) + 4 (n + 1) + 2 n + 4 n, whatever the
     stored layout; the offset-aligned layout stores no column index, so there
     they are an effective rate that can exceed the copy peak, and `stored_*`
-    give the rate over the bytes the product streams (padded values,
-    slice-column bases, row pointers, x and y).  Offset-aligned matrices of
-    constant coefficients (this benchmark's) are multiplied from row patterns:
-    the product then streams x, y and a byte for 8 rows, and the short lists of
-    the rows off the patterns (not counted); it is bound by instruction issue,
-    not by HBM."""
+    give the rate over the bytes the product streams (what the library reports
+    that it reads of the matrix, x and y).  Offset-aligned matrices whose rows
+    repeat (constant coefficients, this benchmark's) are multiplied from row
+    patterns: the product then streams x, y, a byte for 8 rows and the short
+    lists of the rows off the patterns; it is bound by instruction issue, and
+    its `frac` is of those bytes.  The library says which kernel runs."""
     n, nnz = A.shape[0], A.nnz
     info, _ = solver.info()
     x = torch.randn(n, dtype=torch.float32, device="cuda").to(torch.float16)
@@ -266,18 +266,20 @@ def spmv_roofline(solver, A, torch, F):
     aligned = info.index_bits == 0
     csr = info.slice_height == 0
     h = info.slice_height or 32
-    nslices = (n + h - 1) // h
-    idx_bytes = (info.nnz_padded // h) * 4 if aligned else info.nnz_padded * 4
-    # rows from which the library uses the patterns (148 SMs)
-    pattern = aligned and n >= 148 * (2048 if h == 64 else 1024)
-    stored = n * 6 + n // 8 if pattern else alg if csr else info.nnz_padded * 2 + idx_bytes + 4 * (nslices + 1) + n * 2 + n * 4
+    product = solver.product(F.F16, F.F16)
+    pattern = product["kernel"] == "patterns"
+    stored = product["matrix_bytes"] + n * 2 + n * 4
     peak, src = measured_peak()
     achieved = alg / dt / 1e9
+    # the counters were read on the 192^3 stencil's product (128^3, by rows)
+    traffic = None if csr or product["kernel"] == "rows" or n != 192 ** 3 else profiled_traffic(aligned, h, pattern)
     if csr:
         kern = "k_csr_group<__half,__half,EpiStore<float>,1024> (CSR, fp16 A, fp16 x, fp32 y)"
     elif pattern:
         kern = (f"k_sell_pattern<__half,__half,EpiStore<float>> (row patterns of the {h}-row offset-aligned slices, "
                 "fp16 A, fp16 x, fp32 y)")
+    elif product["kernel"] == "rows":
+        kern = "thread-a-row product (short rows or a small packed matrix, fp16 A, fp16 x, fp32 y)"
     elif h == 64:
         kern = "k_sell64<__half,__half,EpiStore<float>,32,1,32> (64-row offset-aligned slices, fp16 A, fp16 x, fp32 y)"
     elif aligned:
@@ -287,7 +289,7 @@ def spmv_roofline(solver, A, torch, F):
         kern = (f"k_sell_cfg<__half,__half,EpiStore<float>,24,2,16,int> (SELL-32 sigma={info.sigma}, fp16 A, fp16 x, "
                 "fp32 y)")
     return {"kernel": kern, "bound": "issue" if pattern else "hbm", "achieved": round(achieved, 1), "peak": peak, "peak_source": src,
-            "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None if csr else profiled_traffic(aligned, h, pattern),
+            "unit": "GB/s", "frac": round((stored / dt / 1e9 if pattern else achieved) / peak, 4), "traffic": traffic,
             "algorithmic_bytes": alg, "effective_rate": aligned, "stored_bytes": stored,
             "stored_achieved": round(stored / dt / 1e9, 1), "stored_frac": round(stored / dt / 1e9 / peak, 4),
             "launch_us": round(dt * 1e6, 2)}

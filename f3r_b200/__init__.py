@@ -239,6 +239,11 @@ def _torch_dt(t):
     return {torch.float64: F64, torch.float32: F32, torch.float16: F16}[t.dtype]
 
 
+def _product(i) -> dict:
+    return dict(kernel=("slices", "csr", "rows", "patterns")[i.kernel], matrix_bytes=i.matrix_bytes,
+                listed_rows=i.listed_rows)
+
+
 class Sell:
     """Device SELL-32-sigma matrix (f3r_sell) -- CoefficientMatrix::operate /
     compute_residual on device tensors."""
@@ -262,6 +267,14 @@ class Sell:
         i = _capi.SellInfo()
         check(lib().f3r_sell_info_get(self._h, C.byref(i)))
         return i
+
+    def product(self, val_t, in_t=None) -> dict:
+        """the kernel that products with these types take (vectors on 16-byte
+        boundaries): "slices", "csr", "rows" or "patterns", the matrix bytes
+        one reads, and for patterns the rows that follow none"""
+        i = _capi.ProductInfo()
+        check(lib().f3r_sell_product_info(self._h, val_t, val_t if in_t is None else in_t, C.byref(i)))
+        return _product(i)
 
     def operate(self, x, y, val_t=None) -> None:
         """y = A x; val_t defaults to the vector type of x (fp16 for fp16 x)."""
@@ -381,6 +394,12 @@ class Solver:
         d = C.c_int32()
         check(lib().f3r_solver_info(self._h, C.byref(i), C.byref(d)))
         return d.value == 2
+
+    def product(self, val_t, in_t=None, columns: int = 1) -> dict:
+        """Sell.product of the solver's matrix; columns: the width of a block of right-hand sides"""
+        i = _capi.ProductInfo()
+        check(lib().f3r_solver_product_info(self._h, val_t, val_t if in_t is None else in_t, columns, C.byref(i)))
+        return _product(i)
 
     def operate(self, x, y, val_t=None) -> None:
         """y = A x with the solver's own device matrix (storage order P A P^T)."""

@@ -65,6 +65,10 @@ class TuneEntry(C.Structure):
                 ("gbs_algorithmic", C.c_double)]
 
 
+class ProductInfo(C.Structure):
+    _fields_ = [("kernel", C.c_int32), ("listed_rows", C.c_int32), ("matrix_bytes", C.c_int64)]
+
+
 COND_FN = C.CFUNCTYPE(C.c_int, C.c_int32, C.c_double, C.c_void_p)
 
 _vp = C.c_void_p
@@ -98,6 +102,7 @@ SIGNATURES = {
     "f3r_context_synchronize": (C.c_int, [_vp]),
     "f3r_sell_create": (C.c_int, [_vp, C.POINTER(CSR), C.c_int32, C.c_int32, C.c_int32, _pp]),
     "f3r_sell_info_get": (C.c_int, [_vp, C.POINTER(SellInfo)]),
+    "f3r_sell_product_info": (C.c_int, [_vp, C.c_int, C.c_int, C.POINTER(ProductInfo)]),
     "f3r_sell_destroy": (None, [_vp]),
     "f3r_sell_tune": (C.c_int, [_vp, C.c_int, C.c_int32, C.POINTER(TuneEntry), C.c_int32, C.POINTER(C.c_int32)]),
     "f3r_sell_operate": (C.c_int, [_vp, C.c_int, C.c_int, _vp, C.c_int, _vp]),
@@ -114,6 +119,7 @@ SIGNATURES = {
                                   C.POINTER(C.c_int64), C.POINTER(_vp), C.POINTER(C.c_int64), COND_FN, _vp,
                                   C.POINTER(Result)]),
     "f3r_solver_info": (C.c_int, [_vp, C.POINTER(SellInfo), C.POINTER(C.c_int32)]),
+    "f3r_solver_product_info": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int32, C.POINTER(ProductInfo)]),
     "f3r_solver_operate": (C.c_int, [_vp, C.c_int, C.c_int, _vp, C.c_int, _vp]),
     "f3r_solver_destroy": (None, [_vp]),
     "f3r_solver_create_factors": (C.c_int, [_vp, C.POINTER(CSR), C.POINTER(Params), C.POINTER(CSR), C.POINTER(CSR),

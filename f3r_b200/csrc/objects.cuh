@@ -121,6 +121,7 @@ struct DeviceSell {
   float *v32 = nullptr;
   __half *v16 = nullptr;
   int dtypes = 0;
+  int64_t index_bytes = 0;  // of columns or slot bases, slice or row starts
   // 32, 16, or 0 (offset-aligned slices, mixed with explicit ones or not)
   int index_bits() const { return (xoff || (cbase && !dcol)) ? 0 : dcol ? 16 : 32; }
   DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, uw, pat}; }
@@ -199,12 +200,9 @@ inline Status launch_direct_packed(Context &c, const V *val, const DevSell &A, c
   return F3R_SUCCESS;
 }
 
-// false where the windows of x do not fit an SM or x is not on a 16-byte boundary
 template <typename V, typename X, typename Epi>
-inline bool launch_pattern(Context &c, const V *val, const DevPattern &d, const X *x, const Epi &epi) {
-  if (reinterpret_cast<uintptr_t>(x) % 16) return false;
+inline void launch_pattern(Context &c, const V *val, const DevPattern &d, const X *x, const Epi &epi) {
   const PatShape p = pattern_shape(d.a, d.warps, sizeof(X), sizeof(PatRun<V>));
-  if (p.stages == 0) return false;
   PatArgs a = d.a;
   a.stages = p.stages;
   a.tail_tile = pattern_tail(a, 16 / (int64_t)sizeof(X));
@@ -213,40 +211,55 @@ inline bool launch_pattern(Context &c, const V *val, const DevPattern &d, const 
   a.rest = PatRest(a.ntiles, a.ngroups, d.warps, grid);
   launch_k(c, k_sell_pattern<V, X, Epi>, (unsigned)grid, (d.warps + 1) * 32, p.smem, c.stream, a, d.tab(val),
            d.vals(val), x, epi, epi_vec4(epi) ? 1 : 0, c.err);
-  return true;
+}
+
+// The kernel that a product takes (x16: x on a 16-byte boundary).  Short rows and
+// small packed matrices: a thread a row (direct.cuh; two rows a lane pay off with
+// fp16 values on 64-row slices, one set of bases, once there is more than one wave
+// of rows: 37.7 -> 33.2 us at 200^3, 1.8 -> 2.1 at 32^3; small packed matrices are
+// one wave of rows, half of one in fp64, whose rows take twice the registers: at
+// 64^3 the bulk kernel is ahead there, 15.6 against 16.9 us).  Repeating rows:
+// patterns (pattern.cuh), from pattern_rows on and where the windows of x fit an SM.
+enum class SellRoute { uniform, short_mixed, short_packed, small_packed, patterns, csr, slices64, slices };
+template <typename V, typename X> inline SellRoute sell_route(const Context &c, const DevSell &A, bool x16) {
+  const bool packed = !A.rptr && !A.cbase && !A.xoff && !A.dcol, all_aligned = A.cbase && !A.xoff && !A.dcol;
+  const int64_t wave = (int64_t)c.sm_count * kDirectResident;
+  if (all_aligned && (A.uw == 4 || A.uw == 8)) return SellRoute::uniform;
+  if (A.max_width <= kDirectShort && (all_aligned || A.xoff)) return SellRoute::short_mixed;
+  if (packed && A.max_width <= kDirectShort) return SellRoute::short_packed;
+  if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave)) return SellRoute::small_packed;
+  if (A.pat && x16 && A.n >= pattern_rows(c.sm_count, A.height, sizeof(V)) &&
+      pattern_shape(A.pat->a, A.pat->warps, sizeof(X), sizeof(PatRun<V>)).stages > 0)
+    return SellRoute::patterns;
+  return A.rptr ? SellRoute::csr : A.height == 64 ? SellRoute::slices64 : SellRoute::slices;
 }
 
 template <typename V, typename X, typename Epi>
 inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
   if (A.nslices == 0) return F3R_SUCCESS;
-  const bool packed = !A.rptr && !A.cbase && !A.xoff && !A.dcol, all_aligned = A.cbase && !A.xoff && !A.dcol;
-  // short rows: thread-a-row kernels (direct.cuh).  Two rows a lane pay off with fp16 values on 64-row
-  // slices (one set of bases) once there is more than one wave of rows: 37.7 -> 33.2 us at 200^3, 1.8 -> 2.1 at 32^3
-  const int64_t wave = (int64_t)c.sm_count * kDirectResident;
-  if (all_aligned && (A.uw == 4 || A.uw == 8)) {
-    if (A.height == 32) return launch_direct_aligned<V, X, Epi, 32, 1>(c, val, A, x, epi);
-    if (sizeof(V) == 2 && A.n > wave) return launch_direct_aligned<V, X, Epi, 64, 2>(c, val, A, x, epi);
-    return launch_direct_aligned<V, X, Epi, 64, 1>(c, val, A, x, epi);
+  const SellRoute route = sell_route<V, X>(c, A, reinterpret_cast<uintptr_t>(x) % 16 == 0);
+  switch (route) {
+    case SellRoute::uniform:
+      if (A.height == 32) return launch_direct_aligned<V, X, Epi, 32, 1>(c, val, A, x, epi);
+      if (sizeof(V) == 2 && A.n > (int64_t)c.sm_count * kDirectResident)
+        return launch_direct_aligned<V, X, Epi, 64, 2>(c, val, A, x, epi);
+      return launch_direct_aligned<V, X, Epi, 64, 1>(c, val, A, x, epi);
+    case SellRoute::short_mixed:
+      if (A.height == 64) return launch_direct_mixed<V, X, Epi, 64>(c, val, A, x, epi);
+      return launch_direct_mixed<V, X, Epi, 32>(c, val, A, x, epi);
+    case SellRoute::short_packed: return launch_direct_packed<V, X, Epi, 4>(c, val, A, x, epi);
+    case SellRoute::small_packed: return launch_direct_packed<V, X, Epi, 8>(c, val, A, x, epi);
+    default: break;
   }
-  if (A.max_width <= kDirectShort && (all_aligned || A.xoff)) {  // mixed form, or slices of 4 and 8 slots
-    if (A.height == 64) return launch_direct_mixed<V, X, Epi, 64>(c, val, A, x, epi);
-    return launch_direct_mixed<V, X, Epi, 32>(c, val, A, x, epi);
-  }
-  if (packed && A.max_width <= kDirectShort) return launch_direct_packed<V, X, Epi, 4>(c, val, A, x, epi);
-  // small packed matrices: one wave of rows (fp64's take twice the registers: half a wave; at 64^3 the bulk kernel is
-  // ahead there, 15.6 against 16.9 us)
-  if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave)) return launch_direct_packed<V, X, Epi, 8>(c, val, A, x, epi);
   F3R_TRY((sell_attr<V, X, Epi>(c)));
-  if (A.pat && A.n >= pattern_rows(c.sm_count, A.height, sizeof(V)) && launch_pattern(c, val, *A.pat, x, epi)) {
-    CUDA_TRY(cudaGetLastError());
-    return F3R_SUCCESS;
-  }
-  if (A.height == 64) {
+  if (route == SellRoute::patterns) {
+    launch_pattern(c, val, *A.pat, x, epi);
+  } else if (route == SellRoute::slices64) {
     using C64 = Sell64Cfg<V>;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(A.nslices, C64::WARPS), c.sm_count));
     launch_k(c, k_sell64<V, X, Epi, C64::WARPS, C64::STAGES, C64::KC>, grid, C64::WARPS * 32, sell64_smem_bytes<V>(),
              c.stream, val, A, x, epi, c.err);
-  } else if (A.rptr) {
+  } else if (route == SellRoute::csr) {
     const unsigned grid = (unsigned)cdiv(A.nslices, kCsrWarps);
     if (A.max_width * 32 <= kCsrShort)
       launch_k(c, k_csr_group<V, X, Epi, kCsrShort>, grid, kCsrWarps * 32, kCsrWarps * csr_tile_bytes<V, kCsrShort>(),

@@ -71,6 +71,7 @@ struct Layout {
   std::vector<uint8_t> blk, live;
   std::vector<int32_t> irow, iptr, icol;
   std::vector<double> ival;
+  int32_t listed = 0;  // rows off their block's pattern
 };
 
 // the runs of a pattern; false where its offsets do not increase or are too many
@@ -305,6 +306,7 @@ static bool layout(const SellHost &h, int sm_count, Layout &o) {
   std::vector<int32_t> rest;
   for (int64_t r = 0; r < n; r++)
     if (off[r]) rest.push_back((int32_t)r);
+  o.listed = (int32_t)rest.size();
   auto width = [&](int32_t r) { return h.sptr[r / h.height + 1] - h.sptr[r / h.height]; };
   std::stable_sort(rest.begin(), rest.end(), [&](int32_t x, int32_t y) { return width(x) < width(y); });
   std::vector<int32_t> &irow = o.irow, &iptr = o.iptr;
@@ -347,6 +349,8 @@ Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d
   DevPattern &p = *dp;
   p.a = o.a;
   p.warps = o.warps;
+  p.listed_rows = o.listed;
+  p.listed_entries = (int64_t)o.icol.size();
   uint8_t *bd = nullptr, *ld = nullptr;
   int32_t *rd = nullptr, *pd = nullptr, *cd = nullptr;
   F3R_TRY(put(c, p, &bd, o.blk.data(), o.blk.size()));

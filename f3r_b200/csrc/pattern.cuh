@@ -360,6 +360,8 @@ struct DevPattern {
   PatArgs a{};
   int warps = 0;
   PatArgs ab{};  // for tiles of one block (patblock.cuh)
+  int32_t listed_rows = 0;     // off their block's pattern
+  int64_t listed_entries = 0;  // of their lists, padding included
   // the patterns' records, for a's tiles and for ab's
   PatRun<double> *t64[2] = {nullptr, nullptr};
   PatRun<float> *t32[2] = {nullptr, nullptr};
@@ -368,6 +370,10 @@ struct DevPattern {
   float *v32 = nullptr;
   __half *v16 = nullptr;
   std::vector<void *> allocs;
+  // what a product reads of the matrix, with values of sv bytes
+  int64_t bytes(size_t sv) const {
+    return listed_entries * (int64_t)(sv + 4) + a.ngroups * (int64_t)(32 * 4 + 4) + a.nblk * (int64_t)33;
+  }
   const PatRun<double> *tab(const double *, int i = 0) const { return t64[i]; }
   const PatRun<float> *tab(const float *, int i = 0) const { return t32[i]; }
   const PatRun<__half> *tab(const __half *, int i = 0) const { return t16[i]; }

@@ -385,6 +385,11 @@ Status upload_sell(Context &c, const SellHost &h, int dtype_mask, bool scatter_p
     F3R_TRY(c.alloc((void **)&d.perm, (size_t)std::max(h.n, 1) * 4));
     CUDA_TRY(cudaMemcpyAsync(d.perm, h.perm.data(), (size_t)h.n * 4, cudaMemcpyHostToDevice, c.stream));
   }
+  d.index_bytes = 4 * (int64_t)(h.nslices + 1);
+  if (!h.xoff.empty() || h.aligned_all)
+    d.index_bytes += 4 * (int64_t)(h.cbase.size() + h.nslices + 1 + (h.aligned_all ? 0 : h.col.size() + h.nslices));
+  else if (!h.dcol.empty()) d.index_bytes += 2 * (int64_t)np + 4 * (int64_t)(h.cbase.size() + h.nslices + 1);
+  else d.index_bytes += 4 * (int64_t)np;
   double *tmp64 = nullptr;
   F3R_TRY(c.alloc((void **)&tmp64, np * 8));
   CUDA_TRY(cudaMemcpyAsync(tmp64, h.val.data(), np * 8, cudaMemcpyHostToDevice, c.stream));
@@ -420,6 +425,7 @@ Status upload_csr(Context &c, const f3r_csr &a, int dtype_mask, DeviceSell &d) {
   d.sigma = 1;
   d.nnz = a.nnz;
   d.nnz_pad = a.nnz;
+  d.index_bytes = 4 * ((int64_t)n + 1 + a.nnz);
   d.dtypes = dtype_mask;
   int32_t mw = 0;
   for (int32_t i = 0; i < n; i++) mw = std::max(mw, a.rptr[i + 1] - a.rptr[i]);
@@ -687,19 +693,22 @@ Status launch_block64(Context &c, const V *val, const DevSell &A, const X *x, co
   return F3R_SUCCESS;
 }
 // K-column product from row patterns (fp16 and fp32 values: fp64's windows leave one block an SM, 124 against 111 us at
-// 81^3 and 8 columns): false where the windows do not fit an SM
+// 81^3 and 8 columns), where the windows fit an SM
+inline bool block_patterns(const DevSell &A, size_t sv, size_t sx, int K) {
+  if (!A.pat || sv == 8) return false;
+  return pattern_shape(A.pat->ab, kPatWarps, sx * K, sv == 2 ? sizeof(PatRun<__half>) : sizeof(PatRun<float>)).stages > 0;
+}
 template <typename V, typename X, typename Epi, int K>
-bool launch_pattern_block(Context &c, const V *val, const DevPattern &d, const X *x, const Epi &epi) {
+void launch_pattern_block(Context &c, const V *val, const DevPattern &d, const X *x, const Epi &epi) {
   const PatShape p = pattern_shape(d.ab, kPatWarps, sizeof(X) * K, sizeof(PatRun<V>));
-  if (p.stages == 0 || reinterpret_cast<uintptr_t>(x) % 16) return false;
   PatArgs a = d.ab;
   a.stages = p.stages;
   a.tail_tile = pattern_tail(a, std::max<int64_t>(1, 16 / (int64_t)(sizeof(X) * K)));
   const int64_t work = std::max<int64_t>(a.ntiles, cdiv(a.ngroups, kPatWarps));
   const int grid = (int)std::min<int64_t>(work, (int64_t)c.sm_count * std::min(p.ctas, 3));
   a.rest = PatRest(a.ntiles, a.ngroups, kPatWarps, grid);
-  launch_k(c, k_pattern_block<V, X, Epi, K>, (unsigned)grid, (kPatWarps + 1) * 32, p.smem, c.stream, a, d.tab(val, 1), d.vals(val), x, epi, c.err);
-  return true;
+  launch_k(c, k_pattern_block<V, X, Epi, K>, (unsigned)grid, (kPatWarps + 1) * 32, p.smem, c.stream, a, d.tab(val, 1),
+           d.vals(val), x, epi, c.err);
 }
 template <typename V, typename X, typename Epi, int K>
 Status launch_block(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi, bool attr_only = false) {
@@ -707,7 +716,8 @@ Status launch_block(Context &c, const V *val, const DevSell &A, const X *x, cons
   if constexpr (sizeof(V) < 8) {
     if (attr_only) {
       CUDA_TRY(cudaFuncSetAttribute(k_pattern_block<V, X, Epi, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    } else if (A.pat && launch_pattern_block<V, X, Epi, K>(c, val, *A.pat, x, epi)) {
+    } else if (block_patterns(A, sizeof(V), sizeof(X), K) && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
+      launch_pattern_block<V, X, Epi, K>(c, val, *A.pat, x, epi);
       CUDA_TRY(cudaGetLastError());
       return F3R_SUCCESS;
     }
@@ -2246,6 +2256,36 @@ Status solver_solve_multi(f3r_solver *s, int32_t nrhs, const double *b, int64_t 
   CUDA_TRY(cudaSetDevice(s->s->ctx->device));
   return s->s->solve_multi(nrhs, b, ldb, x, ldx, cond, user, results);
 }
+
+// what launch_sell (columns = 1) or launch_block would run on d
+static Status product_info(const Context &c, const DeviceSell &d, f3r_dtype val_t, f3r_dtype in_t, int32_t columns,
+                           f3r_product_info &o) {
+  if (val_t < F3R_F64 || val_t > F3R_F16 || !(d.dtypes & (1 << val_t)))
+    return fail(F3R_ERROR_INVALID_VALUE, "matrix holds no copy of that value type");
+  if (!(in_t == val_t || (val_t == F3R_F16 && in_t == F3R_F32)))
+    return fail(F3R_ERROR_UNSUPPORTED, "unsupported (val, in) type combination");
+  if (columns < 1 || columns > kMaxBlock || (columns & (columns - 1)))
+    return fail(F3R_ERROR_INVALID_VALUE, "columns: 1, 2, 4, 8 or 16");
+  const DevSell A = d.view();
+  const size_t sv = val_t == F3R_F64 ? 8 : val_t == F3R_F32 ? 4 : 2, sx = in_t == F3R_F64 ? 8 : in_t == F3R_F32 ? 4 : 2;
+  SellRoute r = SellRoute::slices;
+  if (columns > 1) r = block_patterns(A, sv, sx, columns) ? SellRoute::patterns : SellRoute::slices;
+  else if (val_t == F3R_F64) r = sell_route<double, double>(c, A, true);
+  else if (val_t == F3R_F32) r = sell_route<float, float>(c, A, true);
+  else if (in_t == F3R_F32) r = sell_route<__half, float>(c, A, true);
+  else r = sell_route<__half, __half>(c, A, true);
+  o = f3r_product_info{};
+  o.kernel = r == SellRoute::patterns ? F3R_PRODUCT_PATTERNS
+             : r == SellRoute::csr    ? F3R_PRODUCT_CSR
+             : r == SellRoute::slices || r == SellRoute::slices64 ? F3R_PRODUCT_SLICES : F3R_PRODUCT_ROWS;
+  if (r == SellRoute::patterns) {
+    o.listed_rows = d.pat->listed_rows;
+    o.matrix_bytes = d.pat->bytes(sv);
+  } else {
+    o.matrix_bytes = d.nnz_pad * (int64_t)sv + d.index_bytes;
+  }
+  return F3R_SUCCESS;
+}
 }  // namespace f3r
 
 // ===========================================================================
@@ -2476,6 +2516,10 @@ f3r_status f3r_sell_info_get(const f3r_sell *m, f3r_sell_info *info) {
   info->index_bits = m->d.index_bits();
   return F3R_SUCCESS;
 }
+f3r_status f3r_sell_product_info(const f3r_sell *m, f3r_dtype val_t, f3r_dtype in_t, f3r_product_info *info) {
+  if (!m || !info) return fail(F3R_ERROR_INVALID_VALUE, "null argument");
+  return product_info(*m->ctx, m->d, val_t, in_t, 1, *info);
+}
 void f3r_sell_destroy(f3r_sell *m) {
   if (!m) return;
   if (cudaSetDevice(m->ctx->device) != cudaSuccess) return;  // runtime shutting down: left to the exit
@@ -2624,6 +2668,13 @@ f3r_status f3r_solver_info(const f3r_solver *s, f3r_sell_info *a_info, int32_t *
   }
   if (precond_diagonal) *precond_diagonal = s->s->precond_diag ? (s->s->diag_unit ? 2 : 1) : 0;
   return F3R_SUCCESS;
+}
+f3r_status f3r_solver_product_info(const f3r_solver *s, f3r_dtype val_t, f3r_dtype in_t, int32_t columns,
+                                   f3r_product_info *info) {
+  if (!s || !info) return fail(F3R_ERROR_INVALID_VALUE, "null argument");
+  if (columns > 1 && (s->s->mm || !s->s->block_ok()))
+    return fail(F3R_ERROR_UNSUPPORTED, "this solver takes its right-hand sides one by one, or is a batch");
+  return product_info(*s->s->ctx, s->s->A, val_t, in_t, columns, *info);
 }
 f3r_status f3r_solver_operate(f3r_solver *s, f3r_dtype val_t, f3r_dtype in_t, const void *in, f3r_dtype out_t,
                               void *out) {

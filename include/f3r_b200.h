@@ -317,11 +317,27 @@ f3r_status f3r_sell_compute_residual(f3r_sell *m, f3r_dtype val_t, f3r_dtype rhs
                                      const void *rhs, f3r_dtype in_t, const void *in,
                                      f3r_dtype res_t, void *res);
 
+/* The kernel that products with a matrix take, for given types (vectors on
+ * 16-byte boundaries).  All give the same sums. */
+typedef enum f3r_product_kernel {
+  F3R_PRODUCT_SLICES = 0,   /* slices streamed through shared memory */
+  F3R_PRODUCT_CSR = 1,      /* CSR rows, a warp 32 of them */
+  F3R_PRODUCT_ROWS = 2,     /* a thread a row: short rows, small packed matrices */
+  F3R_PRODUCT_PATTERNS = 3  /* row patterns: offset-aligned matrices whose rows repeat */
+} f3r_product_kernel;
+typedef struct f3r_product_info {
+  int32_t kernel;           /* f3r_product_kernel */
+  int32_t listed_rows;      /* PATTERNS: rows that follow no pattern and are read entry by entry */
+  int64_t matrix_bytes;     /* what one product reads of the stored matrix */
+} f3r_product_info;
+f3r_status f3r_sell_product_info(const f3r_sell *m, f3r_dtype val_t, f3r_dtype in_t, f3r_product_info *info);
+
 /* One launch shape of the SELL SpMV and its measured time (f3r_sell_tune). */
 typedef struct f3r_tune_entry {
   int32_t warps, stages, kc;  /* warps per CTA, bulk-copy stages per warp, columns per copy */
   int32_t index_bits;         /* 32 or 16 (the matrix's index form) */
-  int32_t is_default;         /* 1 for the shape the library launches */
+  int32_t is_default;         /* 1 for the shape the library launches where the product streams the
+                                 slices (f3r_sell_product_info says whether it does) */
   int32_t reserved;
   double microseconds;        /* mean time of one product out = A x */
   double gbs_algorithmic;     /* (nnz*(s_val+4) + 4(n+1) + n*s_x + n*s_y) / time */
@@ -383,6 +399,10 @@ f3r_status f3r_solver_solve(f3r_solver *s, const double *b, double *x, f3r_cond_
  * W^T and Z are both diagonal, 2 when moreover every fp16 value of both is
  * exactly 1 and the Richardson kernels take the constant (diag_load = 0) */
 f3r_status f3r_solver_info(const f3r_solver *s, f3r_sell_info *a_info, int32_t *precond_diagonal);
+/* f3r_sell_product_info of the solver's matrix; columns: the width of a block
+ * of right-hand sides (1, 2, 4, 8 or 16) */
+f3r_status f3r_solver_product_info(const f3r_solver *s, f3r_dtype val_t, f3r_dtype in_t, int32_t columns,
+                                   f3r_product_info *info);
 /* Several right-hand sides: column k of B (b + k * ldb) is solved into
  * column k of X (x + k * ldx), x holding the initial guesses; ldb, ldx >= n;
  * host or device pointers; results (may be NULL) gets one entry per column.

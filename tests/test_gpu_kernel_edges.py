@@ -171,3 +171,56 @@ def test_patterns_and_streamed_kernels_agree_on_non_finite_x(ctx, kw):
         torch.cuda.synchronize()
         assert np.array_equal(ya.cpu().numpy(), yo.cpu().numpy(), equal_nan=True), vt
     S.close()
+
+
+def _rows(per_sm):
+    return per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def test_the_library_reports_the_kernel_that_a_product_takes(ctx):
+    """the kernels either side of each rule, and what the patterns cannot take:
+    varying coefficients, short rows, too few rows"""
+    nz = -(-_rows(1024) // (54 * 53))  # half a wave of rows and up
+    A = F.stencil27(54, 53, nz, 2, 0.5).scale()
+    n = A.shape[0]
+    for kw, want in ((dict(aligned=True), ("patterns",) * 3), (dict(aligned=True, height=64), ("patterns", "patterns", "slices")),
+                     (dict(csr=True), ("csr",) * 3), (dict(), ("slices", "rows", "rows")),
+                     (dict(aligned=True, sigma=256), ("slices",) * 3)):
+        S = F.Sell(ctx, A, **kw)
+        got = tuple(S.product(vt)["kernel"] for vt in (F.F64, F.F32, F.F16))
+        assert got == want, kw
+        S.close()
+    r, i, v = A.arrays()
+    S = F.Sell(ctx, F.HostMatrix.from_csr(r, i, v * np.random.default_rng(0).uniform(1, 2, len(v)), n), aligned=True)
+    p = S.product(F.F16)
+    assert p["kernel"] == "slices" and p["matrix_bytes"] >= S.info().nnz_padded * 2
+    S.close()
+    few = F.Sell(ctx, F.stencil27(54, 53, nz - 1, 2, 0.5).scale(), aligned=True)
+    assert few.product(F.F32)["kernel"] == ("patterns" if 54 * 53 * (nz - 1) >= _rows(1024) else "slices")
+    few.close()
+    S = F.Sell(ctx, F.diffusion7(32, 32, 32, 1.5, 3.0, 1).scale(), aligned=True)
+    assert S.product(F.F16, F.F32)["kernel"] == "rows" and S.product(F.F16)["listed_rows"] == 0
+    with pytest.raises(F.F3RError):
+        S.product(F.F32, F.F16)
+    S.close()
+
+
+@pytest.mark.parametrize("K", [2, 4, 8, 16])
+@pytest.mark.parametrize("variant,kw", [(2, dict(sell_align=1)), (1, dict(sell_align=1, sell_c=64))])
+def test_block_solves_from_patterns_are_the_single_solves(ctx, K, variant, kw):
+    """K columns from row patterns, rows that are no multiple of a 16-byte unit's
+    and a ragged last block: every column its single solve bit for bit"""
+    A = F.stencil27(54, 53, -(-_rows(1024) // (54 * 53)), variant, 0.5).scale()
+    n = A.shape[0]
+    S = F.Solver(ctx, A, rel_tol=1e-10, **kw)
+    for vt, xt in ((F.F16, F.F16), (F.F32, F.F32)):
+        p = S.product(vt, xt, columns=K)
+        assert p["kernel"] == "patterns" and 0 < p["listed_rows"] < n // 2
+    B = np.stack([F.random_uniform(k, -1.0, 1.0, n) for k in range(K)])
+    Y = np.zeros_like(B)
+    rb = S.solve_multi(B, Y)
+    for k in range(K):
+        y = np.zeros(n)
+        r = S.solve(B[k], y)
+        assert r.is_solved and r.res_iter == rb[k].res_iter and np.array_equal(y, Y[k]), k
+    S.close()
