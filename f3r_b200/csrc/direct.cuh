@@ -6,8 +6,7 @@
 // and come here (launch_sell's rule):
 //  * short rows (at most kDirectShort stored columns: 7-point matrices, SDAINV
 //    factors), where a 32-row slice of 4 columns is a 256-byte copy;
-//  * small matrices with packed rows of any length, whose rows are all resident
-//    at once: the bulk kernel's time is then one warp's chain of waits.
+//  * small matrices with packed rows, whose rows are all resident at once: the bulk kernel's time is then one warp's chain of waits.
 // Every thread issues the loads of its row before it uses any of them (in an
 // offset-aligned slice the row's values are contiguous, 8 to 64 bytes), and the
 // SM holds 40 to 64 warps of them.  What bounds it is the latency of the two
@@ -30,6 +29,17 @@ namespace f3r {
 constexpr int kDirectThreads = 256;
 constexpr int kDirectShort = 8;       // widest row of the short form
 constexpr int kDirectResident = 2048;  // rows of a small matrix per SM: one wave of threads
+// Values and columns of a small matrix: sv bytes an entry and 4 for its column.
+// Plain loads pay off while the matrix stays in the 126 MB L2 beside x from one
+// product to the next; the bulk kernel streams past it.  Short fp32 rows (more than
+// half a wave of them) may take a little more.  Bulk kernel -> thread a row, us a
+// product: 150,000 x 80 fp16 (72 MB) 16.5 -> 14.4, 20,000 x 500 fp32 (80 MB) 43 -> 27,
+// 160,000 x 90 fp16 (86 MB) 20.6 -> 22.6, 110,000 x 140 fp16 (92 MB) 17.6 -> 24.5, 20,000 x
+// 1,000 fp16 (120 MB) 71 -> 131; 300,000 x 40 fp32 (96 MB) 20.4 -> 16.5, x 56 (134 MB) 26.0
+// -> 28.4, x 64 fp16 (115 MB) 22.4 -> 28.7.
+inline bool direct_bytes_fit(int64_t entries, size_t sv, int64_t n, int64_t wave) {
+  return entries * (int64_t)(sv + 4) <= (sv == 4 && n * 2 > wave ? 97000000 : 80000000);
+}
 
 // N consecutive values (4 or 8, from a multiple of N) in accesses of up to 32 bytes, not kept in L1
 template <typename V, int N> __device__ __forceinline__ void ld_row(const V *p, V (&o)[N]) {

@@ -124,7 +124,7 @@ struct DeviceSell {
   int64_t index_bytes = 0;  // of columns or slot bases, slice or row starts
   // 32, 16, or 0 (offset-aligned slices, mixed with explicit ones or not)
   int index_bits() const { return (xoff || (cbase && !dcol)) ? 0 : dcol ? 16 : 32; }
-  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, uw, pat}; }
+  DevSell view() const { return DevSell{col, dcol, cbase, cbptr, xoff, sptr, perm, n, ncols, nslices, rptr, height, max_width, nnz_pad, uw, pat}; }
   void release() {
     cudaFree(col); cudaFree(sptr); cudaFree(perm); cudaFree(cbase); cudaFree(cbptr); cudaFree(dcol);
     cudaFree(xoff);
@@ -218,7 +218,8 @@ inline void launch_pattern(Context &c, const V *val, const DevPattern &d, const 
 // fp16 values on 64-row slices, one set of bases, once there is more than one wave
 // of rows: 37.7 -> 33.2 us at 200^3, 1.8 -> 2.1 at 32^3; small packed matrices are
 // one wave of rows, half of one in fp64, whose rows take twice the registers: at
-// 64^3 the bulk kernel is ahead there, 15.6 against 16.9 us).  Repeating rows:
+// 64^3 the bulk kernel is ahead there, 15.6 against 16.9 us, and small enough for
+// L2, direct_bytes_fit).  Repeating rows:
 // patterns (pattern.cuh), from pattern_rows on and where the windows of x fit an SM.
 enum class SellRoute { uniform, short_mixed, short_packed, small_packed, patterns, csr, slices64, slices };
 template <typename V, typename X> inline SellRoute sell_route(const Context &c, const DevSell &A, bool x16) {
@@ -227,7 +228,9 @@ template <typename V, typename X> inline SellRoute sell_route(const Context &c, 
   if (all_aligned && (A.uw == 4 || A.uw == 8)) return SellRoute::uniform;
   if (A.max_width <= kDirectShort && (all_aligned || A.xoff)) return SellRoute::short_mixed;
   if (packed && A.max_width <= kDirectShort) return SellRoute::short_packed;
-  if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave)) return SellRoute::small_packed;
+  if (packed && A.n <= (sizeof(V) == 8 ? wave / 2 : wave) &&
+      direct_bytes_fit(A.nnz_pad, sizeof(V), A.n, wave))
+    return SellRoute::small_packed;
   if (A.pat && x16 && A.n >= pattern_rows(c.sm_count, A.height, sizeof(V)) &&
       pattern_shape(A.pat->a, A.pat->warps, sizeof(X), sizeof(PatRun<V>)).stages > 0)
     return SellRoute::patterns;

@@ -68,6 +68,7 @@ struct DevSell {
   const int32_t *rptr;    // CSR storage: row pointers (col holds the CSR indices), else nullptr
   int32_t height;         // slice height: 32, or 64 (64-row aligned slices, k_sell64)
   int32_t max_width;      // widest slice
+  int64_t nnz_pad;        // stored entries
   int32_t uw;             // the width of every slice where they are all alike (s starts at s * uw), else 0
   const struct DevPattern *pat;  // host side: the rows' patterns where a few cover the matrix (pattern.cuh), else nullptr
 };

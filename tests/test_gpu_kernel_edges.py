@@ -205,6 +205,28 @@ def test_the_library_reports_the_kernel_that_a_product_takes(ctx):
     S.close()
 
 
+@pytest.mark.parametrize("width,dtype,want", [(64, F.F16, "rows"), (200, F.F16, "slices"), (64, F.F32, "rows"),
+                                              (200, F.F64, "slices")])
+def test_long_packed_rows_are_streamed(ctx, width, dtype, want):
+    """100,000 rows: a matrix that stays in L2 is worked a thread a row, one that
+    does not is streamed, as every packed matrix of long rows once was"""
+    n = 100000
+    c = (np.arange(n)[:, None] + np.arange(width) * 3) % n
+    c.sort(1)
+    v = np.random.default_rng(4).standard_normal(n * width)
+    r, i = (np.arange(n + 1) * width).astype(np.int32), c.ravel().astype(np.int32)
+    S = F.Sell(ctx, F.HostMatrix.from_csr(r, i, v, n), dtypes=(dtype,))
+    assert S.product(dtype)["kernel"] == want
+    dt, ov = {F.F64: (np.float64, O.DT_F64), F.F32: (np.float32, O.DT_F32), F.F16: (np.float16, O.DT_F16)}[dtype]
+    x = np.random.default_rng(5).standard_normal(n).astype(dt)
+    y = torch.from_numpy(np.zeros_like(x)).cuda()
+    S.operate(torch.from_numpy(x).cuda(), y, val_t=dtype)
+    torch.cuda.synchronize()
+    want_y = O.spmv(r, i, v, x, ov, ov, O.DT_F64 if dtype == F.F64 else O.DT_F32)
+    assert np.array_equal(y.cpu().numpy().view(np.uint8), want_y.view(np.uint8))
+    S.close()
+
+
 @pytest.mark.parametrize("K", [2, 4, 8, 16])
 @pytest.mark.parametrize("variant,kw", [(2, dict(sell_align=1)), (1, dict(sell_align=1, sell_c=64))])
 def test_block_solves_from_patterns_are_the_single_solves(ctx, K, variant, kw):
