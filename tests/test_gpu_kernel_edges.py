@@ -40,6 +40,33 @@ def test_block_ilu_solve_is_the_oracles(ctx, grid, blocks, sigma):
     assert c != 0 and np.all(np.abs(x / c - want) <= 4 * 2.0 ** -24 * np.abs(want))
 
 
+@pytest.mark.parametrize("grid,blocks", [((32, 32, 32), 32768), ((32, 32, 32), 4096), ((24, 25, 27), 300), ((40, 40, 1), 33)])
+def test_small_ilu_blocks_cost_what_they_hold(ctx, grid, blocks):
+    """blocks of one row and of a few: the device memory of a solver does not
+    grow with their number (32,768 rows: the matrix and its vectors take under 32
+    MB, both factors at 4 words for each they need 12 MB), and a block solve is the oracle's"""
+    A = F.stencil27(*grid, 1, 0.5).scale()
+    n = A.shape[0]
+    r, i, v = A.arrays()
+    b = np.where(F.random_uniform(3, 0.0, 1.0, n) < 0.5, -1.0, 1.0)
+    L, U = O.ilu0_bj(O.Mat.from_csr(r, i, v), blocks)
+    h = (b / np.sqrt(n)).astype(np.float16)
+    kw = dict(precond=F.PRECOND_ILU0_BJ, ilu_blocks=blocks, m2=1, m3=0, m4=1, static_weight=1.0)
+    F.Solver(ctx, A, **kw).close()  # kernels loaded
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    S = F.Solver(ctx, A, **kw)
+    assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+    x = np.zeros(n)
+    S.solve(b, x, cond=lambda it, e: it >= 1)
+    S.close()
+    # b's entries are +-1: h is b over a factor that fp16 rounds, the same for every row
+    want = O.trsv(U, True, O.trsv(L, False, h, prod_fma=True), prod_fma=True).astype(np.float64)
+    c = np.dot(x, want) / np.dot(want, want)
+    ulp = 4 * 2.0 ** -24 if float(h[0] * b[0]) ** 2 * n == 1.0 else 2.0 ** -10
+    assert c != 0 and np.all(np.abs(x / c - want) <= ulp * np.abs(want).max())
+
+
 @pytest.mark.parametrize("kind,grid,kw", [
     ("7pt", (64, 3, 2), dict(aligned=True, height=64)), ("7pt", (67, 5, 3), dict(aligned=True)),  # ragged last slices
     ("7pt", (67, 71, 64), dict(aligned=True, height=64)),  # more than one wave: two rows a lane
