@@ -167,7 +167,7 @@ Status put_values(Context &c, DevPattern &p, const Layout &o, PatRun<V> *(&tab)[
     for (const Run &r : q.runs) flat.insert(flat.end(), r.v, r.v + 3);
   std::vector<V> rv;
   F3R_TRY(rounded<V>(c, flat, rv));
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < (o.ab.ntiles > 0 ? 2 : 1); i++) {
     const std::vector<int32_t> &soff = i ? o.soffb : o.soff;
     std::vector<PatRun<V>> t((size_t)p.a.np * p.a.stride);
     std::memset((void *)t.data(), 0, t.size() * sizeof(PatRun<V>));
@@ -300,8 +300,11 @@ static bool layout(const SellHost &h, int sm_count, Layout &o) {
   o.ab = a;
   o.ab.tile = kPatBlock;
   o.ab.ntiles = nblk;
-  if (!windows(pats, a, o.soff) || !windows(pats, o.ab, o.soffb)) return false;
+  if (!windows(pats, a, o.soff)) return false;
   if (pattern_shape(a, o.warps, 2, sizeof(PatRun<__half>)).stages == 0) return false;
+  // offsets a block or more apart take a window each there (a 27-point stencil on lines of 258 rows and
+  // more has 9): the K-column products then stream the matrix, the others keep their 3
+  if (!windows(pats, o.ab, o.soffb)) o.ab.ntiles = 0;
   // the other rows, grouped by width
   std::vector<int32_t> rest;
   for (int64_t r = 0; r < n; r++)

@@ -359,7 +359,7 @@ __global__ void __launch_bounds__((kPatWarps + 1) * 32, sizeof(V) == 8 ? 2 : 4)
 struct DevPattern {
   PatArgs a{};
   int warps = 0;
-  PatArgs ab{};  // for tiles of one block (patblock.cuh)
+  PatArgs ab{};  // for tiles of one block (patblock.cuh); ntiles = 0: too many windows
   int32_t listed_rows = 0;     // off their block's pattern
   int64_t listed_entries = 0;  // of their lists, padding included
   // the patterns' records, for a's tiles and for ab's

@@ -695,7 +695,7 @@ Status launch_block64(Context &c, const V *val, const DevSell &A, const X *x, co
 // K-column product from row patterns (fp16 and fp32 values: fp64's windows leave one block an SM, 124 against 111 us at
 // 81^3 and 8 columns), where the windows fit an SM
 inline bool block_patterns(const DevSell &A, size_t sv, size_t sx, int K) {
-  if (!A.pat || sv == 8) return false;
+  if (!A.pat || sv == 8 || A.pat->ab.ntiles == 0) return false;
   return pattern_shape(A.pat->ab, kPatWarps, sx * K, sv == 2 ? sizeof(PatRun<__half>) : sizeof(PatRun<float>)).stages > 0;
 }
 template <typename V, typename X, typename Epi, int K>

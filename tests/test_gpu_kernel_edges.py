@@ -273,3 +273,29 @@ def test_block_solves_from_patterns_are_the_single_solves(ctx, K, variant, kw):
         r = S.solve(B[k], y)
         assert r.is_solved and r.res_iter == rb[k].res_iter and np.array_equal(y, Y[k]), k
     S.close()
+
+
+@pytest.mark.parametrize("nx,block", [(257, "patterns"), (258, "slices"), (400, "slices")])
+def test_patterns_of_long_grid_lines(ctx, nx, block):
+    """lines longer than a pattern's block: the single-column product keeps the
+    patterns where the K-column one has too many windows; both bit for bit"""
+    ny, nz = 40, -(-_rows(1024) // (nx * 40))
+    A = F.stencil27(nx, ny, nz, 2, 0.5).scale()
+    r, i, v = A.arrays()
+    n = A.shape[0]
+    S = F.Solver(ctx, A, rel_tol=1e-10, sell_align=1)
+    assert S.product(F.F16)["kernel"] == "patterns" and S.product(F.F16, columns=8)["kernel"] == block
+    x = np.random.default_rng(2).standard_normal(n)
+    for vt, dt, ov, oacc in ((F.F64, np.float64, O.DT_F64, O.DT_F64), (F.F32, np.float32, O.DT_F32, O.DT_F32),
+                             (F.F16, np.float16, O.DT_F16, O.DT_F32)):
+        xd = torch.from_numpy(x.astype(dt)).cuda()
+        y = torch.zeros_like(xd)
+        S.operate(xd, y, val_t=vt)
+        torch.cuda.synchronize()
+        assert np.array_equal(y.cpu().numpy(), O.spmv(r, i, v, x.astype(dt), ov, ov, oacc)), vt
+    B = np.stack([F.random_uniform(k, -1.0, 1.0, n) for k in range(2)])
+    Y, y = np.zeros_like(B), np.zeros(n)
+    S.solve_multi(B, Y)
+    S.solve(B[1], y)
+    assert np.array_equal(y, Y[1])
+    S.close()
