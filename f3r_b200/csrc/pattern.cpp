@@ -140,20 +140,24 @@ template <typename T> Status put(Context &c, DevPattern &p, T **d, const T *h, s
   return F3R_SUCCESS;
 }
 
+struct Temp {
+  void *p = nullptr;
+  ~Temp() { cudaFree(p); }
+};
+
 // v in type T as the device rounds the matrix's values
 template <typename T> Status rounded(Context &c, const std::vector<double> &v, std::vector<T> &o) {
-  double *d = nullptr;
-  T *t = nullptr;
+  Temp a, b;
   o.resize(v.size());
-  F3R_TRY(c.alloc((void **)&d, v.size() * 8));
-  F3R_TRY(c.alloc((void **)&t, v.size() * sizeof(T)));
+  F3R_TRY(c.alloc(&a.p, v.size() * 8));
+  F3R_TRY(c.alloc(&b.p, v.size() * sizeof(T)));
+  double *d = static_cast<double *>(a.p);
+  T *t = static_cast<T *>(b.p);
   CUDA_TRY(cudaMemcpyAsync(d, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c.stream));
   launch_k(c, k_convert_vals<T>, c.ew_grid((int64_t)v.size()), kEwThreads, 0, c.stream, (const double *)d, t,
            (int64_t)v.size());
   CUDA_TRY(cudaMemcpyAsync((void *)o.data(), t, v.size() * sizeof(T), cudaMemcpyDeviceToHost, c.stream));
   CUDA_TRY(cudaStreamSynchronize(c.stream));
-  cudaFree(d);
-  cudaFree(t);
   return F3R_SUCCESS;
 }
 
@@ -188,14 +192,14 @@ Status put_values(Context &c, DevPattern &p, const Layout &o, PatRun<V> *(&tab)[
   F3R_TRY(c.alloc((void **)val, std::max<size_t>(ival.size(), 1) * sizeof(V)));
   p.allocs.push_back((void *)*val);
   if (!ival.empty()) {
-    double *d = nullptr;
-    F3R_TRY(c.alloc((void **)&d, ival.size() * 8));
+    Temp a;
+    F3R_TRY(c.alloc(&a.p, ival.size() * 8));
+    double *d = static_cast<double *>(a.p);
     CUDA_TRY(cudaMemcpyAsync(d, ival.data(), ival.size() * 8, cudaMemcpyHostToDevice, c.stream));
     launch_k(c, k_convert_vals<V>, c.ew_grid((int64_t)ival.size()), kEwThreads, 0, c.stream, (const double *)d, *val,
              (int64_t)ival.size());
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(c.stream));
-    cudaFree(d);
   }
   return F3R_SUCCESS;
 }
@@ -345,9 +349,7 @@ static bool layout(const SellHost &h, int sm_count, Layout &o) {
   return true;
 }
 
-Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d) {
-  Layout o;
-  if (!layout(h, c.sm_count, o)) return F3R_SUCCESS;
+static Status upload_pattern(Context &c, const Layout &o, int dtype_mask, DeviceSell &d) {
   auto dp = std::make_unique<DevPattern>();
   DevPattern &p = *dp;
   p.a = o.a;
@@ -378,6 +380,16 @@ Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d
   if (dtype_mask & (1 << F3R_F16)) F3R_TRY(put_values<__half>(c, p, o, p.t16, &p.v16));
   CUDA_TRY(cudaStreamSynchronize(c.stream));
   d.pat = dp.release();
+  return F3R_SUCCESS;
+}
+
+// A matrix works without its patterns: where the device has no room for them, it does.
+Status make_pattern(Context &c, const SellHost &h, int dtype_mask, DeviceSell &d) {
+  Layout o;
+  if (!layout(h, c.sm_count, o)) return F3R_SUCCESS;
+  const Status s = upload_pattern(c, o, dtype_mask, d);
+  if (s != F3R_ERROR_OUT_OF_MEMORY) return s;
+  clear_stale_error();
   return F3R_SUCCESS;
 }
 

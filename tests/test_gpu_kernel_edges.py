@@ -299,3 +299,34 @@ def test_patterns_of_long_grid_lines(ctx, nx, block):
     S.solve(B[1], y)
     assert np.array_equal(y, Y[1])
     S.close()
+
+
+def test_a_matrix_that_leaves_no_room_for_patterns_is_streamed(ctx):
+    """the patterns are an extra: with device memory for the matrix and not for
+    the lists of the rows off them, the matrix works as it did without"""
+    A = F.stencil27(12, 400, 400, 2, 0.5).scale()  # lists of a sixth of the rows
+    n = A.shape[0]
+    x = torch.from_numpy(np.random.default_rng(6).standard_normal(n)).cuda()
+    y, z = torch.zeros_like(x), torch.zeros_like(x)
+    F.Sell(ctx, A, aligned=True).close()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    S = F.Sell(ctx, A, aligned=True)
+    S.operate(x, y)
+    ctx.synchronize()
+    p, total = S.product(F.F64), free - torch.cuda.mem_get_info()[0]
+    assert p["kernel"] == "patterns" and p["listed_rows"] > n // 8
+    S.close()
+    # value copies of 8, 4 and 2 bytes and one of columns
+    lists = p["listed_rows"] * 28 * (8 + 4 + 2 + 4)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (total - lists // 2), dtype=torch.uint8, device="cuda")
+    try:
+        S = F.Sell(ctx, A, aligned=True)
+        assert S.product(F.F64)["kernel"] == "slices"
+        S.operate(x, z)
+        ctx.synchronize()
+        S.close()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert torch.equal(y, z)
