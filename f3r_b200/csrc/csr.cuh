@@ -14,7 +14,10 @@
 // warps that the hardware schedules as others finish, one tile of shared memory a
 // warp, and tiles of kCsrShort entries where every group fits them (rows of at
 // most 8 entries: 64 warps an SM; 128^3 7-point, fp32: 27.5 us, 52.4 with
-// kCsrWide), of kCsrWide otherwise.  Against 24 persistent warps an SM with a
+// kCsrWide), of kCsrMid where every group fits those (rows of 9 to 16; 10^6 x 10,
+// kCsrWide -> kCsrMid: fp32 24.4 -> 18.5 us, fp64 45.3 -> 32.9) and for fp64 rows of
+// up to 64, whose wide tiles leave 16 warps an SM (300,000 x 40 61.4 -> 55.3, x 64
+// 159.9 -> 152.7; x 100 113.9 -> 148), of kCsrWide otherwise.  Against 24 persistent warps an SM with a
 // two-stage ring of 512 entries: 27-point, fp16, 40^3 7.4 -> 4.1 us, 64^3 17.5 ->
 // 9.4, 128^3 109 -> 74; 7-point 64^3 6.5 -> 4.4, 200^3 147 -> 100.
 #pragma once
@@ -23,7 +26,7 @@
 
 namespace f3r {
 
-constexpr int kCsrWide = 1024, kCsrShort = 256;  // entries a tile
+constexpr int kCsrWide = 1024, kCsrMid = 512, kCsrShort = 256;  // entries a tile
 constexpr int kCsrWarps = 4;                     // warps a block
 constexpr int kCsrPad = 16;                      // elements of padding after the value and index arrays
 

@@ -178,6 +178,12 @@ inline void launch_sell_one(Context &c, const V *val, const DevSell &A, const X 
            sell_smem_bytes<V, CI>(), c.stream, val, A, x, epi, c.err);
 }
 
+template <typename V, typename X, typename Epi, int T>
+inline void launch_csr(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
+  launch_k(c, k_csr_group<V, X, Epi, T>, (unsigned)cdiv(A.nslices, kCsrWarps), kCsrWarps * 32,
+           kCsrWarps * csr_tile_bytes<V, T>(), c.stream, val, A, x, epi);
+}
+
 template <typename V, typename X, typename Epi, int H, int R>
 inline Status launch_direct_aligned(Context &c, const V *val, const DevSell &A, const X *x, const Epi &epi) {
   launch_k(c, k_sell_direct_aligned<V, X, Epi, H, R>, (unsigned)cdiv(cdiv(A.n, 32 * R) * 32, kDirectThreads),
@@ -263,13 +269,9 @@ inline Status launch_sell(Context &c, const V *val, const DevSell &A, const X *x
     launch_k(c, k_sell64<V, X, Epi, C64::WARPS, C64::STAGES, C64::KC>, grid, C64::WARPS * 32, sell64_smem_bytes<V>(),
              c.stream, val, A, x, epi, c.err);
   } else if (route == SellRoute::csr) {
-    const unsigned grid = (unsigned)cdiv(A.nslices, kCsrWarps);
-    if (A.max_width * 32 <= kCsrShort)
-      launch_k(c, k_csr_group<V, X, Epi, kCsrShort>, grid, kCsrWarps * 32, kCsrWarps * csr_tile_bytes<V, kCsrShort>(),
-               c.stream, val, A, x, epi);
-    else
-      launch_k(c, k_csr_group<V, X, Epi, kCsrWide>, grid, kCsrWarps * 32, kCsrWarps * csr_tile_bytes<V, kCsrWide>(),
-               c.stream, val, A, x, epi);
+    if (A.max_width * 32 <= kCsrShort) launch_csr<V, X, Epi, kCsrShort>(c, val, A, x, epi);
+    else if (A.max_width * 32 <= kCsrMid || (sizeof(V) == 8 && A.max_width <= 64)) launch_csr<V, X, Epi, kCsrMid>(c, val, A, x, epi);
+    else launch_csr<V, X, Epi, kCsrWide>(c, val, A, x, epi);
   } else if (A.xoff) launch_sell_one<V, X, Epi, AlignedIdx>(c, val, A, x, epi);
   else if (A.cbase && !A.dcol) launch_sell_one<V, X, Epi, AllAlignedIdx>(c, val, A, x, epi);
   else if (A.dcol) launch_sell_one<V, X, Epi, uint16_t>(c, val, A, x, epi);

@@ -159,6 +159,27 @@ def test_csr_tiles_bitexact(ctx, n, lo, hi):
     S.close()
 
 
+@pytest.mark.parametrize("n,lo,hi", [(97, 16, 16), (101, 0, 17), (130, 64, 64), (129, 1, 65)])
+def test_csr_middle_tiles_bitexact(ctx, n, lo, hi):
+    """groups that fill a tile of 512 entries or take several, either side of the rows it is chosen for"""
+    rng = np.random.default_rng(hi)
+    cnt = rng.integers(lo, hi + 1, n)
+    cnt[n // 2] = hi
+    r = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    i = np.concatenate([np.sort(rng.choice(n, c, replace=False)) for c in cnt]).astype(np.int32)
+    v = rng.standard_normal(len(i))
+    S = F.Sell(ctx, F.HostMatrix.from_csr(r, i, v, n), csr=True)
+    x = rng.standard_normal(n)
+    for vt, dt, ov in ((F.F64, np.float64, O.DT_F64), (F.F32, np.float32, O.DT_F32), (F.F16, np.float16, O.DT_F16)):
+        xd = torch.from_numpy(x.astype(dt)).cuda()
+        y = torch.zeros_like(xd)
+        S.operate(xd, y, val_t=vt)
+        torch.cuda.synchronize()
+        want = O.spmv(r, i, v, x.astype(dt), ov, ov, O.DT_F64 if vt == F.F64 else O.DT_F32)
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), want.view(np.uint8)), vt
+    S.close()
+
+
 @pytest.mark.parametrize("grid", [(13, 11, 7), (32, 32, 32), (70, 69, 63), (97, 90, 71)])
 @pytest.mark.parametrize("m2,m3", [(8, 4), (3, 8), (5, 0)])
 def test_single_column_levels_are_the_block_kernels(ctx, grid, m2, m3):
