@@ -78,12 +78,14 @@ __global__ void k_trsv_bj(IluTri T, const __half *__restrict__ in, __half *__res
 // the block), padded to the part's longest row so that no lane branches.  The copy engine keeps kBjStages chunks
 // ahead of the sweep, so a level costs only shared-memory latencies; a row's
 // packed data is read one and two parts ahead, which leaves the gather of y,
-// the multiply-add chain and one barrier between two levels.  W warps sweep (one,
-// without any block barrier, where levels hold up to 32 rows on average); the
-// other warps only load and store the block's vector.
-// 64^3, 112 blocks, both factors (272 levels): 49 us, where one launch a factor
-// reading it from L2 level by level took 453 us; the solve 15.9 ms against 59.7.
-// What is left is the sweep's own chain, 0.17 us a level.
+// the multiply-add chain and one barrier between two levels.  W warps sweep: one,
+// without any block barrier, where levels hold up to 32 rows on average or where
+// whole chunks would be half empty; the other warps only load and store the block's
+// vector.
+// 64^3, 112 blocks, both factors (272 levels): 41 us, where one launch a factor
+// reading it from L2 level by level took 453 us.  What is left is the sweep's own
+// chain, 0.15 us a level.  (A row's groups are not unrolled where one warp sweeps: 41
+// against 45 us; several warps: 222 against 211 us at 16 blocks.)
 // The in-place vector y holds the right-hand side, then L^-1 in, then the
 // result; the terms and roundings of a row are k_trsv_bj's.
 // ---------------------------------------------------------------------------

@@ -21,12 +21,15 @@
 // Every row's multiply-adds are the stored layout's, in its order, padding
 // included (a zero times the last x, which only a non-finite x can see), so the
 // sums are the streamed kernels' bit for bit.
-// What bounds it now is issue (380 warp instructions for 128 rows of 27 entries,
-// 108 of them multiply-adds) and, below about a million rows, 5 us of set-up
-// and first-tile latency.  27-point stencil, 64-row slices, us a product,
-// streamed -> here:  fp16 x fp16  81^3 9.1 -> 5.9, 128^3 28.9 -> 14.4, 160^3 51.8 -> 20.0;
-// fp32  128^3 40.7 -> 17.4, 160^3 75.7 -> 26.8;  fp64  128^3 75.0 -> 29.9, 160^3 147 -> 73.
-// The 192^3 solve: 93.7 -> 53.9 ms.
+// What bounds it now is issue (397 warp instructions for 128 rows of 27 entries,
+// 108 of them multiply-adds, the other rows' lists included) and, below about a
+// million rows, 5 us of set-up and first-tile latency.  27-point stencil, us a product,
+// streamed (64-row slices) -> here:  fp16 x fp16  81^3 9.1 -> 5.9, 128^3 28.9 -> 14.4, 192^3
+// 86.5 -> 33.5;  fp32  128^3 40.7 -> 18.5, 192^3 130 -> 42;  fp64  128^3 75.0 -> 32.8, 192^3
+// 267 -> 100.7.  The 192^3 solve took 93.3 ms with streamed products and 44.3 with these
+// and the kernels of blas1.cuh.
+// Setting the patterns up reads every row twice on the host: 0.28 s of the 3 s that a
+// 192^3 matrix takes to lay out.
 #pragma once
 
 #include <algorithm>

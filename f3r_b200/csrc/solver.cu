@@ -1270,8 +1270,11 @@ template <int K> struct Engine {
   // Kernels of single-column solves are set up while their predecessors run
   // (Context::overlap) where a launch is a good part of a kernel: systems of up to
   // kOverlapRows rows, and short rows (many kernels of one wave after another).
-  // 16^3 27-point 1,531 -> 1,437 us, 40^3 2,461 -> 2,313, 7-point 50^3 3,162 ->
-  // 2,877, 90^3 10,609 -> 10,133.  Blocks of an early kernel go where room is left,
+  // In order -> early, us an outer step, packed: 27-point 14^3 740 -> 694, 28^3 777 ->
+  // 704, 40^3 822 -> 761; 7-point 16^3 950 -> 832, 50^3 1,026 -> 920, 90^3 2,155 -> 2,047,
+  // 128^3 4,929 -> 4,774, 160^3 8,833 -> 8,706 (0 to 14% over 12 27-point grids of up to
+  // 64,000 rows and 15 7-point ones, in four layouts; one of the 106 pairs, 64^3 packed,
+  // read 2% slower).  Blocks of an early kernel go where room is left,
   // which unbalances kernels sized for one even wave: 27-point 64^3 4,630 -> 4,912,
   // row patterns at 100^3 8,418 -> 9,714, CSR at 40^3 2,644 -> 4,908; those launch
   // in order.
